@@ -19,9 +19,10 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgila_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["gila.cu", "matvec.cu", "matvec_c128.cu", "matvec_c64.cu", "noalloc.cu", "slab.cu", "kerbuild.cu",
-           "solver.cu", "server.cu"]
-HEADERS = ["fft.cuh", "fft_ct.cuh", "matvec.cuh", "matvec_impl.cuh", "internal.h", "solver.h"]
+SOURCES = ["matvec_c128.cu", "matvec_c64.cu", "gila.cu", "matvec.cu", "noalloc.cu", "slab.cu", "kerbuild.cu",
+           "solver.cu", "server.cu", *(f"matvec_mx_{k}.cu" for k in range(8))]
+HEADERS = ["fft.cuh", "fft_ct.cuh", "fft_mx.cuh", "matvec.cuh", "matvec_impl.cuh", "matvec_mx.cuh",
+           "matvec_mx_impl.cuh", "passes.cuh", "internal.h", "solver.h"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
