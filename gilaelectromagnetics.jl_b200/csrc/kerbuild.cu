@@ -24,12 +24,14 @@
 //      dtype, NaN/Inf check.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <vector>
 
 #include "internal.h"
+#include "matvec_mx.cuh"
 
 namespace gila {
 namespace kb {
@@ -86,57 +88,135 @@ struct Tri6 {
   double r[6][3];
 };
 
-__device__ inline void spx(double xp[3][2], double e1, double e2, double x1, double x2) {
-  xp[0][0] = (S3 * (1.0 - e1) - x1) / (2.0 * S3);
-  xp[1][0] = (S3 * (1.0 + e1) - x1) / (2.0 * S3);
-  xp[2][0] = x1 / S3;
-  xp[0][1] = (S3 * (1.0 - e2) - x2) / (2.0 * S3);
-  xp[1][1] = (S3 * (1.0 + e2) - x2) / (2.0 * S3);
-  xp[2][1] = x2 / S3;
-}
-__device__ inline double dist6(const Tri6& t, const double xp[3][2]) {
-  double v[3];
-  for (int d = 0; d < 3; ++d)
-    v[d] = xp[0][0] * t.r[0][d] + xp[1][0] * t.r[1][d] + xp[2][0] * t.r[2][d] -
-           (xp[0][1] * t.r[3][d] + xp[1][1] * t.r[4][d] + xp[2][1] * t.r[5][d]);
-  return sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-}
-__device__ inline double dist3(const Tri6& t, const double xp[3][2]) {
-  double v[3];
-  for (int d = 0; d < 3; ++d)
-    v[d] = xp[0][0] * t.r[0][d] + xp[1][0] * t.r[1][d] + xp[2][0] * t.r[2][d] -
-           (xp[0][1] * t.r[0][d] + xp[1][1] * t.r[1][d] + xp[2][1] * t.r[2][d]);
-  return sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+// Point of a triangle (r0, r1, r2) at (e, x) of the DIRECTFN simplex (spX!,
+// src/glaIntSup.jl): affine, C + De e + Dx x.
+struct Aff {
+  double c[3], e[3], x[3];
+};
+__device__ inline Aff tri_aff(const double (*r)[3]) {
+  Aff a;
+  for (int d = 0; d < 3; ++d) {
+    a.c[d] = 0.5 * (r[0][d] + r[1][d]);
+    a.e[d] = 0.5 * (r[1][d] - r[0][d]);
+    a.x[d] = (r[2][d] - a.c[d]) / S3;
+  }
+  return a;
 }
 
-// subTri (src/glaIntSup.jl:365-379)
-__device__ inline void sub_tri(double l1, double l2, int dir, double& e, double& x) {
-  if (dir == 1) {
-    e = l1;
-    x = l2;
-  } else if (dir == 2) {
-    e = 0.5 * (1.0 - l1 - l2 * S3);
-    x = 0.5 * (S3 + l1 * S3 - l2);
+// Along the innermost variable z of every weak integral the two points move
+// on straight lines, so their difference is A + B z, and the integrand is
+// z^k times the (regularised) kernel at its length.  One kernel value: for a
+// real frequency a sine / cosine pair of the half phase, and e^{i t} - 1 =
+// -2 sin^2(t/2) + 2 i sin(t/2) cos(t/2), which does not cancel at small t; the
+// division by the length is one reciprocal root.  `rq` holds f.x and 1 / (4 pi
+// f.x^2); a frequency with an imaginary part takes scl_ego / scl_ego_n.
+struct RealF {
+  double f, s;
+};
+// (out of line: the registers of its range reduction would count in every
+// kernel below)
+static __device__ __noinline__ double2 sincos_pi_any(double x) {
+  double2 r;
+  sincospi(x, &r.x, &r.y);
+  return r;
+}
+// sin(pi x), cos(pi x).  Phases of up to a quarter half-turn -- every weak
+// integral of cells below 1/8 wavelength -- take the Taylor sums to x^15 and
+// x^16 (the next terms are below 5e-17): 16 multiply-adds instead of the
+// library's range reduction and selects (weak integrals of a cubic cell at
+// intOrd 32: 2.25 -> 2.11 ms).
+__device__ __forceinline__ void sincos_pi(double x, double* sn, double* cs) {
+  if (fabs(x) <= 0.25) {
+    const double y = x * PI, t = y * y;
+    double s = -1.0 / 1307674368000.0, c = 1.0 / 20922789888000.0;
+    s = fma(s, t, 1.0 / 6227020800.0);
+    c = fma(c, t, -1.0 / 87178291200.0);
+    s = fma(s, t, -1.0 / 39916800.0);
+    c = fma(c, t, 1.0 / 479001600.0);
+    s = fma(s, t, 1.0 / 362880.0);
+    c = fma(c, t, -1.0 / 3628800.0);
+    s = fma(s, t, -1.0 / 5040.0);
+    c = fma(c, t, 1.0 / 40320.0);
+    s = fma(s, t, 1.0 / 120.0);
+    c = fma(c, t, -1.0 / 720.0);
+    s = fma(s, t, -1.0 / 6.0);
+    c = fma(c, t, 1.0 / 24.0);
+    c = fma(c, t, -0.5);
+    *sn = fma(s * t, y, y);
+    *cs = fma(c, t, 1.0);
+    return;
+  }
+  const double2 r = sincos_pi_any(x);
+  *sn = r.x;
+  *cs = r.y;
+}
+template <bool RF>
+__device__ __forceinline__ Z ego_line(double r2, bool sng, Z f, RealF rq) {
+  if constexpr (RF) {
+    if (!sng) {
+      double i = rsqrt(r2);
+      double sn, cs;
+      sincos_pi(2.0 * (r2 * i) * rq.f, &sn, &cs);
+      i *= rq.s;
+      return Z{i * cs, i * sn};
+    }
+    if (r2 > 1e-14) {
+      const double i = rsqrt(r2);
+      double sn, cs;
+      sincos_pi((r2 * i) * rq.f, &sn, &cs);
+      const double g = 2.0 * sn * (i * rq.s);
+      return Z{-g * sn, g * cs};
+    }
+    return Z{-0.5 * PI * sqrt(r2), 0.5 / rq.f};  // the limit (scl_ego_n)
   } else {
-    e = 0.5 * (-1.0 - l1 + l2 * S3);
-    x = 0.5 * (S3 - l1 * S3 - l2);
+    const double d = sqrt(r2);
+    return sng ? scl_ego_n(d, f) : scl_ego(d, f);
   }
 }
-// aS (src/glaIntSup.jl:313-332)
-__device__ Z a_s(const Tri6& t, double th1, double thB, double th, int dir, const Consts& q) {
-  double xp[3][2];
-  Z acc{0, 0};
-  double s1, c1;
-  sincos(th1, &s1, &c1);
-  for (int n = 0; n < q.ord; ++n) {
-    double e1, x1, e2, x2;
-    sub_tri(thB, th * s1, dir, e1, x1);
-    const double u = thf(0.0, th, q.x[n]);
-    sub_tri(u * c1 + thB, (th - u) * s1, dir, e2, x2);
-    spx(xp, e1, e2, x1, x2);
-    acc = zadd(acc, zsc(scl_ego_n(dist3(t, xp), q.f), q.w[n] * u));
+
+// aS (src/glaIntSup.jl:313-332).  Both points lie on one triangle, subTri
+// (src/glaIntSup.jl:365-379) is linear and the variable runs over u = th t, so
+// the distance is th t |w| with w fixed by the angle and the sub-triangle
+// (s_dir): the kernel's 1 / d cancels the weight u.
+__device__ inline double s_dir(const Aff& a, double s1, double c1, int dir) {
+  double de, dx;
+  if (dir == 1) {
+    de = -c1;
+    dx = s1;
+  } else if (dir == 2) {
+    de = 0.5 * (c1 - s1 * S3);
+    dx = 0.5 * (-c1 * S3 - s1);
+  } else {
+    de = 0.5 * (c1 + s1 * S3);
+    dx = 0.5 * (c1 * S3 - s1);
   }
-  return zsc(acc, 0.5 * th);
+  double q = 0;
+  for (int d = 0; d < 3; ++d) {
+    const double v = a.e[d] * de + a.x[d] * dx;
+    q += v * v;
+  }
+  return sqrt(q);
+}
+template <bool RF>
+__device__ Z a_s(double wl, double th, const Consts& q, RealF rq) {
+  Z acc{0, 0};
+  for (int n = 0; n < q.ord; ++n) {
+    const double u = thf(0.0, th, q.x[n]), d = u * wl;
+    if constexpr (RF) {
+      if (d > 1e-7) {
+        double sn, cs;
+        sincos_pi(d * rq.f, &sn, &cs);
+        const double g = 2.0 * q.w[n] * sn;
+        acc.x -= g * sn;
+        acc.y += g * cs;
+        continue;
+      }
+      acc = zadd(acc, zsc(Z{-0.5 * PI * d, 0.5 / rq.f}, q.w[n] * (d / rq.s)));  // the limit (scl_ego_n)
+    } else {
+      acc = zadd(acc, zsc(scl_ego_n(d, q.f), q.w[n] * u));
+    }
+  }
+  return zsc(acc, RF ? 0.5 * th * rq.s / wl : 0.5 * th);
 }
 __device__ inline void psi_lim_s(int idf, double& a, double& b) {
   if (idf == 1 || idf == 5 || idf == 6) {
@@ -172,81 +252,92 @@ __device__ inline void eta_lim_s(int idf, double th, double& a, double& b) {
   }
 }
 // nS (src/glaIntSup.jl:201-237): the n-th term (weight included) and its factor
-__device__ inline Z n_s_term(int dir, int idf, double th1, double thB, int n, const Tri6& t, const Consts& q) {
-  double L, fac;
+template <bool RF>
+__device__ inline Z n_s_term(int idf, double s1, double c1, double wl, double thB, int n, const Consts& q, RealF rq) {
+  double L;
   if (idf == 1 || idf == 5) {
-    L = (1.0 - thB) / cos(th1);
-    fac = (1.0 - thB) / (2.0 * cos(th1));
+    L = (1.0 - thB) / c1;
   } else if (idf == 2 || idf == 3) {
-    L = S3 * (1.0 - thB) / sin(th1);
-    fac = S3 * (1.0 - thB) / (2.0 * sin(th1));
+    L = S3 * (1.0 - thB) / s1;
   } else if (idf == 6 || idf == 7) {
-    L = S3 * (1.0 + thB) / sin(th1);
-    fac = S3 * (1.0 + thB) / (2.0 * sin(th1));
+    L = S3 * (1.0 + thB) / s1;
   } else {
-    L = -(1.0 + thB) / cos(th1);
-    fac = -(1.0 + thB) / (2.0 * cos(th1));
+    L = -(1.0 + thB) / c1;
   }
-  return zsc(a_s(t, th1, thB, thf(0.0, L, q.x[n]), dir, q), fac * q.w[n]);
+  return zsc(a_s<RF>(wl, thf(0.0, L, q.x[n]), q, rq), 0.5 * L * q.w[n]);
 }
 
-// spxE! / aE / intNE (src/glaIntSup.jl:283-348,395-411)
-__device__ inline void spx_e(double xp[3][2], double lam, double eta, double thB, double th1, int idf) {
-  double sB, cB, s1, c1;
-  sincos(thB, &sB, &cB);
-  sincos(th1, &s1, &c1);
-  if (idf == 1)
-    spx(xp, eta, lam * cB * c1 - eta, lam * sB, lam * cB * s1);
-  else
-    spx(xp, -eta, -(lam * cB * c1 - eta), lam * sB, lam * cB * s1);
-}
-__device__ Z a_e(const Tri6& t, double lam, double eta, double thB, double th1, int idf, const Consts& q) {
-  double xp[3][2];
+// spxE! / aE / intNE (src/glaIntSup.jl:283-348,395-411): a pair's two
+// triangles and the angles of the current point of the outer sums
+struct EdgeGeo {
+  const double (*v)[3];  // shared: C1 - C2, De1 + De2, Dx1, De2 c1, Dx2 s1
+  double sB, cB, tB, s1, c1;
+};
+template <bool RF>
+__device__ __forceinline__ Z a_e(const EdgeGeo& t, double lam, double eta, double sg, const Consts& q, RealF rq) {
+  // sg 1: points (eta, z sB), (z cB c1 - eta, z cB s1); -1: the same with both
+  // first coordinates negated
+  double A[3], B[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    A[d] = t.v[0][d] + sg * eta * t.v[1][d];
+    B[d] = t.v[2][d] * t.sB - t.cB * (sg * t.v[3][d] + t.v[4][d]);
+  }
   Z acc{0, 0};
+#pragma unroll 1
   for (int n = 0; n < q.ord; ++n) {
     const double z = thf(0.0, lam, q.x[n]);
-    spx_e(xp, z, eta, thB, th1, idf);
-    acc = zadd(acc, zsc(scl_ego_n(dist6(t, xp), q.f), q.w[n] * z * z));
+    const double x = A[0] + B[0] * z, y = A[1] + B[1] * z, w = A[2] + B[2] * z;
+    acc = zadd(acc, zsc(ego_line<RF>(x * x + y * y + w * w, true, q.f, rq), q.w[n] * z * z));
   }
   return zsc(acc, 0.5 * lam);
 }
-__device__ Z int_ne(int n, int idf1, double gam, double thB, double th1, const Tri6& t, int idf2, const Consts& q) {
-  double eta, lam, s1, c1;
-  sincos(th1, &s1, &c1);
+// both orientations (idf 1 and -1) of the n-th term share eta and lam
+template <bool RF>
+__device__ Z int_ne(int n, int idf1, double gam, const EdgeGeo& t, const Consts& q, RealF rq) {
+  double eta, lam;
   if (idf1 == 1) {
     eta = thf(0.0, gam, q.x[n]);
-    lam = S3 * (1 + eta) / (cos(thB) * (s1 + S3 * c1));
+    lam = S3 * (1 + eta) / (t.cB * (t.s1 + S3 * t.c1));
   } else if (idf1 == 2) {
     eta = thf(gam, 1.0, q.x[n]);
-    lam = S3 * (1.0 - fabs(eta)) / sin(thB);
+    lam = S3 * (1.0 - fabs(eta)) / t.sB;
   } else if (idf1 == 3) {
     eta = thf(gam, 1.0, q.x[n]);
-    lam = S3 * (1.0 - fabs(eta)) / (cos(thB) * (s1 - S3 * c1));
+    lam = S3 * (1.0 - fabs(eta)) / (t.cB * (t.s1 - S3 * t.c1));
   } else if (idf1 == 4) {
     eta = thf(0.0, 1.0, q.x[n]);
-    lam = S3 * (1.0 - fabs(eta)) / (cos(thB) * (s1 - S3 * c1));
+    lam = S3 * (1.0 - fabs(eta)) / (t.cB * (t.s1 - S3 * t.c1));
   } else {
     eta = thf(0.0, 1.0, q.x[n]);
-    lam = S3 * (1.0 - eta) / sin(thB);
+    lam = S3 * (1.0 - eta) / t.sB;
   }
-  return a_e(t, lam, eta, thB, th1, idf2, q);
+  Z v{0, 0};
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) v = zadd(v, a_e<RF>(t, lam, eta, h ? -1.0 : 1.0, q, rq));
+  return v;
 }
-// n-th term of nE(idf1, idf2, thB, th1) (src/glaIntSup.jl:239-281), weight included
-__device__ Z n_e_term(int idf1, int idf2, double thB, double th1, int n, const Tri6& t, const Consts& q) {
-  if (idf1 == 1 || idf1 == 2) {
-    double s1, c1;
-    sincos(th1, &s1, &c1);
-    const double gam = (s1 + S3 * c1 - tan(thB)) / (s1 + S3 * c1 + tan(thB));
-    const Z a = int_ne(n, 1, gam, thB, th1, t, idf2, q), b = int_ne(n, 2, gam, thB, th1, t, idf2, q);
-    return zsc(zadd(zsc(b, 0.5), zsc(zsub(a, b), gam * 0.5)), q.w[n]);
+// n-th term of nE(idf1, 1, ...) + nE(idf1, -1, ...) (src/glaIntSup.jl:239-281),
+// weight included
+template <bool RF>
+__device__ Z n_e_term(int idf1, int n, const EdgeGeo& t, const Consts& q, RealF rq) {
+  // (idf1 1, 2: parts 1 and 2 at gam; 3: parts 1 and 3; 4, 5: one part)
+  const bool two = idf1 <= 3;
+  double gam = 1.0;
+  if (idf1 <= 2) {
+    const double k = t.s1 + S3 * t.c1;
+    gam = (k - t.tB) / (k + t.tB);
   } else if (idf1 == 3) {
-    const double gam = S3 / tan(th1);
-    const Z a = int_ne(n, 1, gam, thB, th1, t, idf2, q), b = int_ne(n, 3, gam, thB, th1, t, idf2, q);
-    return zsc(zadd(zsc(b, 0.5), zsc(zsub(a, b), 0.5 * gam)), q.w[n]);
-  } else if (idf1 == 4) {
-    return zsc(int_ne(n, 4, 1.0, thB, th1, t, idf2, q), 0.5 * q.w[n]);
+    gam = S3 * t.c1 / t.s1;
   }
-  return zsc(int_ne(n, 5, 1.0, thB, th1, t, idf2, q), 0.5 * q.w[n]);
+  Z v{0, 0};
+#pragma unroll 1
+  for (int h = 0; h < (two ? 2 : 1); ++h) {
+    const int part = !two ? (idf1 == 4 ? 4 : 5) : h == 0 ? 1 : idf1 == 3 ? 3 : 2;
+    const double w = !two ? 0.5 : h == 0 ? 0.5 * gam : 0.5 - 0.5 * gam;
+    v = zadd(v, zsc(int_ne<RF>(n, part, gam, t, q, rq), w));
+  }
+  return zsc(v, q.w[n]);
 }
 __device__ inline void psi_lim_e(int idf, double& a, double& b) {
   if (idf == 1) {
@@ -283,14 +374,6 @@ __device__ inline void eta_lim_e(int idf, double th, double& a, double& b) {
     b = 0.5 * PI;
   }
 }
-__device__ inline void spx_v(double xp[3][2], double t4, double t3, double tB, double t1) {
-  double sB, cB, s1, c1, s3, c3;
-  sincos(tB, &sB, &cB);
-  sincos(t1, &s1, &c1);
-  sincos(t3, &s3, &c3);
-  spx(xp, t4 * c3 * c1 - 1.0, t4 * s3 * cB - 1.0, t4 * c3 * s1, t4 * s3 * sB);
-}
-
 // One weak item: a triangle pair and its integral type.
 enum { W_S = 0, W_E = 1, W_VS = 2, W_VR = 3 };
 struct WItem {
@@ -312,85 +395,134 @@ __device__ inline Z block_sum(Z v, Z* sh) {
   return s;
 }
 
-// grid: blockIdx.x = outer index of the item's sum; partial[item][outer]
-__global__ void __launch_bounds__(256) k_weak(const WItem* __restrict__ items, int item0, int n_outer,
-                                              const Consts* __restrict__ qp, Z* __restrict__ partial) {
+// One block per (item, outer index of its sum) of the items of one kind (0:
+// self, 1: edge, 2: vertex), item0 .. item0 + nitems - 1 with `outer` blocks
+// each; partial[item][outer].
+//
+// Bound by FP64 arithmetic: 906 M kernel values for three directions at intOrd
+// 32, a third of that where the sides are equal.  All items of a kind in one
+// launch: an item alone has 32 (vertex) to 768 blocks, and one after the other
+// they left most SMs idle.  A kernel per kind, with the pair's geometry in
+// shared memory, holds 76 to 128 registers (one kernel for all: 152, one block
+// per SM, 2.11 ms).  Cubic cell at intOrd 32: 108 launches of 49.7 ms in all,
+// now 0.31 (self) + 0.78 (edge) + 0.25 ms (vertex).
+template <int KIND, bool RF>
+__global__ void __launch_bounds__(256, 2) k_weak(const WItem* __restrict__ items, int item0, int n_outer, int stride,
+                                                 const Consts* __restrict__ qp, Z* __restrict__ partial) {
   __shared__ Consts q;
   __shared__ Z sh[8];
   __shared__ Tri6 t;
+  __shared__ double geo[5][3];
   __shared__ int type;
-  const int item = item0 + blockIdx.y;
+  const int item = item0 + (int)blockIdx.x / n_outer, outer = (int)blockIdx.x % n_outer;
+  for (int i = threadIdx.x; i < (int)(sizeof(Consts) / sizeof(double)); i += blockDim.x)
+    reinterpret_cast<double*>(&q)[i] = reinterpret_cast<const double*>(qp)[i];
   if (threadIdx.x == 0) {
-    q = *qp;
     t = items[item].t;
     type = items[item].type;
   }
   __syncthreads();
   const int n = q.ord;
-  const int outer = blockIdx.x;
+  const RealF rq{q.f.x, 1.0 / (4.0 * PI * q.f.x * q.f.x)};
   Z acc{0, 0};
   double scale = 1.0;
-  if (type == W_S) {
+  if constexpr (KIND == 0) {
     // outer = (k*8 + idf-1)*3 + dir-1 ; inner (it, nn)
     const int dir = outer % 3 + 1, idf = (outer / 3) % 8 + 1, k = outer / 24;
     double pa, pb, ea, eb;
     psi_lim_s(idf, pa, pb);
     const double th = thf(pa, pb, q.x[k]);
     eta_lim_s(idf, th, ea, eb);
+    double s1, c1;
+    sincos(th, &s1, &c1);
+    const double wl = s_dir(tri_aff(t.r), s1, c1, dir);
     for (int p = threadIdx.x; p < n * n; p += blockDim.x) {
       const int it = p / n, nn = p % n;
       const double thB = thf(ea, eb, q.x[it]);
-      acc = zadd(acc, zsc(n_s_term(dir, idf, th, thB, nn, t, q), q.w[it]));
+      acc = zadd(acc, zsc(n_s_term<RF>(idf, s1, c1, wl, thB, nn, q, rq), q.w[it]));
     }
-    scale = 0.25 * q.w[k] * (pb - pa) * (eb - ea) * sin(th);
-  } else if (type == W_E) {
+    scale = 0.25 * q.w[k] * (pb - pa) * (eb - ea) * s1;
+  } else if constexpr (KIND == 1) {
     const int idf = outer % 6 + 1, k = outer / 6;
     double pa, pb, ea, eb;
     psi_lim_e(idf, pa, pb);
     const double thB = thf(pa, pb, q.x[k]);
     eta_lim_e(idf, thB, ea, eb);
+    EdgeGeo g;
+    sincos(thB, &g.s1, &g.c1);  // the outer angle is the inner sums' th1
+    if (threadIdx.x == 0) {
+      const Aff a = tri_aff(t.r), b = tri_aff(t.r + 3);
+      for (int d = 0; d < 3; ++d) {
+        geo[0][d] = a.c[d] - b.c[d];
+        geo[1][d] = a.e[d] + b.e[d];
+        geo[2][d] = a.x[d];
+        geo[3][d] = b.e[d] * g.c1;
+        geo[4][d] = b.x[d] * g.s1;
+      }
+    }
+    __syncthreads();
+    g.v = geo;
     for (int p = threadIdx.x; p < n * n; p += blockDim.x) {
       const int it = p / n, nn = p % n;
       const double thA = thf(ea, eb, q.x[it]);
-      const Z v = zadd(n_e_term(idf, 1, thA, thB, nn, t, q), n_e_term(idf, -1, thA, thB, nn, t, q));
-      acc = zadd(acc, zsc(v, q.w[it] * cos(thA)));
+      sincos(thA, &g.sB, &g.cB);
+      g.tB = g.sB / g.cB;
+      acc = zadd(acc, zsc(n_e_term<RF>(idf, nn, g, q, rq), q.w[it] * g.cB));
     }
     scale = 0.25 * q.w[k] * (pb - pa) * (eb - ea);
   } else {
     const bool sng = type == W_VS;
     const int i3 = outer;
+    // spxV! (src/glaIntSup.jl): points (tx c3 cA - 1, tx c3 sA) and (tx s3 cB
+    // - 1, tx s3 sB) of the two triangles
+    if (threadIdx.x == 0) {
+      const Aff a = tri_aff(t.r), b = tri_aff(t.r + 3);
+      for (int d = 0; d < 3; ++d) {
+        geo[0][d] = t.r[0][d] - t.r[3][d];
+        geo[1][d] = a.e[d];
+        geo[2][d] = a.x[d];
+        geo[3][d] = b.e[d];
+        geo[4][d] = b.x[d];
+      }
+    }
+    __syncthreads();
     for (int p = threadIdx.x; p < n * n; p += blockDim.x) {
       const int i2 = p / n, i1 = p % n;
-      double xp[3][2];
-      const double tA = thf(0.0, PI / 3.0, q.x[i1]);
-      const double LA = 2.0 * S3 / (sin(tA) + S3 * cos(tA));
-      const double tB = thf(0.0, PI / 3.0, q.x[i2]);
-      const double LB = 2.0 * S3 / (sin(tB) + S3 * cos(tB));
+      double sA, cA, sB, cB;
+      sincos(thf(0.0, PI / 3.0, q.x[i1]), &sA, &cA);
+      sincos(thf(0.0, PI / 3.0, q.x[i2]), &sB, &cB);
+      const double LA = 2.0 * S3 / (sA + S3 * cA);
+      const double LB = 2.0 * S3 / (sB + S3 * cB);
       const double at = atan(LB / LA);
-      const double tC = thf(0.0, at, q.x[i3]);
-      double sC, cC, sD, cD;
-      sincos(tC, &sC, &cC);
-      const double tD = thf(at, PI / 2.0, q.x[i3]);
-      sincos(tD, &sD, &cD);
-      Z vc{0, 0}, vd{0, 0};
-      for (int a = 0; a < n; ++a) {
-        const double tx = thf(0.0, LA / cC, q.x[a]);
-        spx_v(xp, tx, tC, tB, tA);
-        const double d = dist6(t, xp);
-        vc = zadd(vc, zsc(sng ? scl_ego_n(d, q.f) : scl_ego(d, q.f), q.w[a] * (tx * tx * tx)));
+      Z v[2];
+      double s3[2], c3[2];
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const double ang = h ? thf(at, PI / 2.0, q.x[i3]) : thf(0.0, at, q.x[i3]);
+        double sn, cs;
+        sincos(ang, &sn, &cs);
+        const double len = h ? LB / sn : LA / cs;
+        double B[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          B[d] = (geo[1][d] * cA + geo[2][d] * sA) * cs - (geo[3][d] * cB + geo[4][d] * sB) * sn;
+        Z s{0, 0};
+#pragma unroll 1
+        for (int a = 0; a < n; ++a) {
+          const double tx = thf(0.0, len, q.x[a]);
+          const double x = geo[0][0] + B[0] * tx, y = geo[0][1] + B[1] * tx, w = geo[0][2] + B[2] * tx;
+          s = zadd(s, zsc(ego_line<RF>(x * x + y * y + w * w, sng, q.f, rq), q.w[a] * (tx * tx * tx)));
+        }
+        v[h] = s;
+        s3[h] = sn;
+        c3[h] = cs;
       }
-      for (int a = 0; a < n; ++a) {
-        const double tx = thf(0.0, LB / sD, q.x[a]);
-        spx_v(xp, tx, tD, tB, tA);
-        const double d = dist6(t, xp);
-        vd = zadd(vd, zsc(sng ? scl_ego_n(d, q.f) : scl_ego(d, q.f), q.w[a] * (tx * tx * tx)));
-      }
-      const Z term = zadd(zsc(zsub(zsc(vc, LA * sC), zsc(vd, LB * cD)), at), zsc(vd, 0.5 * PI * LB * cD));
+      const Z term = zadd(zsc(zsub(zsc(v[0], LA * s3[0]), zsc(v[1], LB * c3[1])), at), zsc(v[1], 0.5 * PI * LB * c3[1]));
       acc = zadd(acc, zsc(term, q.w[i1] * q.w[i2] * q.w[i3]));
     }
   }
   const Z s = block_sum(acc, sh);
-  if (threadIdx.x == 0) partial[(size_t)item * n_outer + outer] = zsc(s, scale);
+  if (threadIdx.x == 0) partial[(size_t)item * stride + outer] = zsc(s, scale);
 }
 
 __device__ inline double cross_norm(const double a[3], const double b[3], const double c[3]) {
@@ -400,13 +532,18 @@ __device__ inline double cross_norm(const double a[3], const double b[3], const 
   return sqrt(x * x + y * y + z * z);
 }
 
-// per item: fixed-order sum of its partials times the Jacobian factor
-__global__ void k_weak_reduce(const WItem* __restrict__ items, int nitems, const int* __restrict__ nout,
-                              const Z* __restrict__ partial, int stride, Z* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nitems) return;
+// per item: fixed-order sum of its partials (one warp) times the Jacobian
+// factor
+__global__ void __launch_bounds__(32) k_weak_reduce(const WItem* __restrict__ items, int ord,
+                                                    const Z* __restrict__ partial, int stride, Z* __restrict__ out) {
+  const int i = blockIdx.x, ty = items[i].type, nout = ty == W_S ? 24 * ord : ty == W_E ? 6 * ord : ord;
   Z s{0, 0};
-  for (int k = 0; k < nout[i]; ++k) s = zadd(s, partial[(size_t)i * stride + k]);
+  for (int k = threadIdx.x; k < nout; k += 32) s = zadd(s, partial[(size_t)i * stride + k]);
+  for (int o = 16; o > 0; o >>= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+  }
+  if (threadIdx.x != 0) return;
   const Tri6& t = items[i].t;
   double jac;
   if (items[i].type == W_S) {
@@ -467,43 +604,51 @@ __device__ Z r_srf_edg_flt(double la, double lb, Z f) {
   return zadd(zsc(zdiv(Z{1.0, 0.0}, zsc(zmul(f, f), 12.0 * PI)), p1), Z{p2 / (64.0 * PI), 0.0});
 }
 
-// wS[3], wE[9], wV[6] from the item sums (layout fixed by weak_items) and the
-// closed forms, scaled by inv = 1/prod(scl) (src/glaInt.jl:75-262, glaGen.jl:115-121)
-__global__ void k_weak_combine(const Z* __restrict__ it, const double* __restrict__ scl, double inv, Z f,
-                               Z* __restrict__ w /* 18 scaled */, Z* __restrict__ wraw /* 18 unscaled */) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double s1 = scl[0], s2 = scl[1], s3 = scl[2];
+// wS[3], wE[9], wV[6] from the item sums (layout fixed by weak_items; uid[k]
+// is the distinct item that item k equals) and the closed forms, scaled by
+// inv = 1/prod(scl) (src/glaInt.jl:75-262, glaGen.jl:115-121).  One warp:
+// lane k < 15 evaluates closed form k.
+__global__ void __launch_bounds__(32) k_weak_combine(const Z* __restrict__ sums, const int* __restrict__ uid,
+                                                     const double* __restrict__ scl, double inv, Z f,
+                                                     Z* __restrict__ w /* 18 scaled */,
+                                                     Z* __restrict__ wraw /* 18 unscaled */) {
+  __shared__ Z cf[15];
+  const double l[3] = {scl[0], scl[1], scl[2]};
+  {
+    // operands (axes) of the self (3), flat-edge (6) and corner (6) forms
+    const signed char op[15][3] = {{1, 2, 0}, {0, 2, 0}, {0, 1, 0}, {2, 1, 0}, {1, 2, 0}, {0, 2, 0}, {2, 0, 0}, {1, 0, 0},
+                                   {0, 1, 0}, {2, 1, 0}, {1, 2, 0}, {0, 2, 1}, {2, 1, 0}, {1, 2, 0}, {0, 2, 1}};
+    const int k = threadIdx.x < 15 ? threadIdx.x : 14;
+    double a[3];
+    for (int d = 0; d < 3; ++d) a[d] = op[k][d] == 0 ? l[0] : op[k][d] == 1 ? l[1] : l[2];
+    Z v;
+    if (k < 3)
+      v = r_srf_slf(a[0], a[1], f);
+    else if (k < 9)
+      v = r_srf_edg_flt(a[0], a[1], f);
+    else
+      v = r_srf_edg_crn(a[0], a[1], a[2], f);
+    if (threadIdx.x < 15) cf[k] = v;
+  }
+  __syncwarp();
+  if (threadIdx.x != 0) return;
+  auto it = [&](int k) { return sums[uid[k]]; };
+  auto sum4 = [&](int k) { return zadd(zadd(zadd(it(k), it(k + 1)), it(k + 2)), it(k + 3)); };
   // items: per dir d (0: dir 3, 1: dir 2, 2: dir 1) -> S block 8 items, E block 16, V block 12
-  auto sdir = [&](int b) {  // wekSDir
-    const Z* p = it + b * 36;
-    Z a = zadd(zadd(zadd(p[0], p[1]), p[2]), p[3]);
-    Z c = zadd(zadd(zadd(p[4], p[5]), p[6]), p[7]);
-    return zsc(zadd(a, c), 0.5);
-  };
-  auto edir = [&](int b, int k) {  // wekEDir value k
-    const Z* p = it + b * 36 + 8 + 4 * k;
-    return zadd(zadd(zadd(p[0], p[1]), p[2]), p[3]);
-  };
-  auto vdir = [&](int b, int k) {  // wekVDir value k
-    const Z* p = it + b * 36 + 24 + 4 * k;
-    return zadd(zadd(zadd(p[0], p[1]), p[2]), p[3]);
-  };
+  auto sdir = [&](int b) { return zsc(zadd(sum4(b * 36), sum4(b * 36 + 4)), 0.5); };  // wekSDir
+  auto edir = [&](int b, int k) { return sum4(b * 36 + 8 + 4 * k); };                   // wekEDir value k
+  auto vdir = [&](int b, int k) { return sum4(b * 36 + 24 + 4 * k); };                  // wekVDir value k
   Z r[18];
-  r[0] = zadd(sdir(0), r_srf_slf(s2, s3, f));
-  r[1] = zadd(sdir(1), r_srf_slf(s1, s3, f));
-  r[2] = zadd(sdir(2), r_srf_slf(s1, s2, f));
-  const Z xxY = zadd(edir(0, 0), r_srf_edg_flt(s3, s2, f)), xxZ = zadd(edir(0, 2), r_srf_edg_flt(s2, s3, f));
-  const Z xyA = zadd(edir(0, 1), r_srf_edg_crn(s3, s2, s1, f)), xzA = zadd(edir(0, 3), r_srf_edg_crn(s2, s3, s1, f));
-  const Z yyZ = zadd(edir(1, 0), r_srf_edg_flt(s1, s3, f)), yyX = zadd(edir(1, 2), r_srf_edg_flt(s3, s1, f));
-  const Z yzA = zadd(edir(1, 1), r_srf_edg_crn(s1, s3, s2, f)), xyB = zadd(edir(1, 3), r_srf_edg_crn(s3, s2, s1, f));
-  const Z zzX = zadd(edir(2, 0), r_srf_edg_flt(s2, s1, f)), zzY = zadd(edir(2, 2), r_srf_edg_flt(s1, s2, f));
-  const Z xzB = zadd(edir(2, 1), r_srf_edg_crn(s2, s3, s1, f)), yzB = zadd(edir(2, 3), r_srf_edg_crn(s1, s3, s2, f));
-  r[3] = xxY;
-  r[4] = xxZ;
-  r[5] = yyX;
-  r[6] = yyZ;
-  r[7] = zzX;
-  r[8] = zzY;
+  for (int b = 0; b < 3; ++b) r[b] = zadd(sdir(b), cf[b]);
+  const Z xyA = zadd(edir(0, 1), cf[9]), xzA = zadd(edir(0, 3), cf[10]);
+  const Z yzA = zadd(edir(1, 1), cf[11]), xyB = zadd(edir(1, 3), cf[12]);
+  const Z xzB = zadd(edir(2, 1), cf[13]), yzB = zadd(edir(2, 3), cf[14]);
+  r[3] = zadd(edir(0, 0), cf[3]);  // xx along y
+  r[4] = zadd(edir(0, 2), cf[4]);  // xx along z
+  r[5] = zadd(edir(1, 2), cf[6]);  // yy along x
+  r[6] = zadd(edir(1, 0), cf[5]);  // yy along z
+  r[7] = zadd(edir(2, 0), cf[7]);  // zz along x
+  r[8] = zadd(edir(2, 2), cf[8]);  // zz along y
   r[9] = zsc(zadd(xyA, xyB), 0.5);
   r[10] = zsc(zadd(xzA, xzB), 0.5);
   r[11] = zsc(zadd(yzA, yzB), 0.5);
@@ -533,217 +678,251 @@ struct PairGeo {
 
 // the 24 face pairs (0-based fp = 6*ft + fs) that feed the six stored
 // components (xx, yy, zz, xy, xz, yz) of srfSum! (src/glaGen.jl:531-555)
-__constant__ int c_pairs[24] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 14, 15, 16, 17, 20, 21, 22, 23, 28, 29, 34, 35};
+#define GILA_PAIRS {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 14, 15, 16, 17, 20, 21, 22, 23, 28, 29, 34, 35}
+__constant__ int c_pairs[24] = GILA_PAIRS;
+__device__ constexpr int kPairs[24] = GILA_PAIRS;
 
-__device__ inline void face_val(const PairGeo& G, int ft, int fs, const double sep[3], const double u[4],
-                                double out[2]) {
-  double v[3];
-  for (int d = 0; d < 3; ++d) {
-    const double tv = G.tf.o[ft][d] + u[2] * G.tf.a[ft][d] + u[3] * G.tf.b[ft][d];
-    const double sv = G.sf.o[fs][d] + u[0] * G.sf.a[fs][d] + u[1] * G.sf.b[fs][d];
-    v[d] = (tv - sv) + sep[d];
-  }
-  const Z z = scl_ego(sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]), G.f);
-  out[0] = z.x;
-  out[1] = z.y;
-}
-
-struct Region {
-  double c[4], h[4], val[2], err[2], errmax;
-  int split;
+// A pair's integrand at u in [0,1]^4: the vector between the two faces' points
+// is o + u0 a0 + u1 a1 + u2 a2 + u3 a3 (source edges negated), the separation
+// of the cells included.
+struct PairLine {
+  double o[3], a[4][3];
 };
+__device__ inline PairLine pair_line(const PairGeo& G, int fp, const double sep[3]) {
+  const int ft = fp / 6, fs = fp % 6;
+  PairLine l;
+  for (int d = 0; d < 3; ++d) {
+    l.o[d] = (G.tf.o[ft][d] - G.sf.o[fs][d]) + sep[d];
+    l.a[0][d] = -G.sf.a[fs][d];
+    l.a[1][d] = -G.sf.b[fs][d];
+    l.a[2][d] = G.tf.a[ft][d];
+    l.a[3][d] = G.tf.b[ft][d];
+  }
+  return l;
+}
+// sclEgo at a squared distance
+template <bool RF>
+__device__ __forceinline__ Z ego_at(double r2, Z f, RealF rq) {
+  if constexpr (RF) return ego_line<true>(r2, false, f, rq);
+  return scl_ego(sqrt(r2), f);
+}
 
 constexpr double GL2 = 0.35856858280031809199064515390793749545;  // sqrt(9/70)
 constexpr double GL4 = 0.94868329805051379959966806332981556011;  // sqrt(9/10)
 constexpr double GL5 = 0.68824720161168529772162873429362352512;  // sqrt(9/19)
 
-// point p of the 57-point Genz-Malik rule: offsets in units of the half-widths
+// The 57-point Genz-Malik rule: points 0 (centre), 1 + 4 i + k (axis i; -l2,
+// +l2, -l4, +l4), 17 .. 40 (two axes at +-l4), 41 .. 56 (all at +-l5), as
+// offsets in units of the half-widths, and the degree-7 and -5 weights.
+constexpr int kGm = 57;
 __device__ inline void gm_point(int p, double off[4]) {
   off[0] = off[1] = off[2] = off[3] = 0.0;
   if (p == 0) return;
-  if (p <= 16) {  // 1 + 4*i + k, k: -l2, +l2, -l4, +l4
+  if (p <= 16) {
     const int q = p - 1, i = q / 4, k = q % 4;
-    off[i] = (k < 2 ? GL2 : GL4) * ((k & 1) ? 1.0 : -1.0);
+    const double v = (k < 2 ? GL2 : GL4) * ((k & 1) ? 1.0 : -1.0);
+    for (int d = 0; d < 4; ++d)
+      if (d == i) off[d] = v;
     return;
   }
   if (p <= 40) {
     const int q = p - 17, pr = q / 4;
-    const int pi[6] = {0, 0, 0, 1, 1, 2}, pk[6] = {1, 2, 3, 2, 3, 3};
-    off[pi[pr]] = GL4 * ((q & 1) ? 1.0 : -1.0);
-    off[pk[pr]] = GL4 * ((q & 2) ? 1.0 : -1.0);
+    const int pi = pr < 3 ? 0 : pr < 5 ? 1 : 2, pk = pr < 3 ? pr + 1 : pr < 5 ? pr - 1 : 3;
+    for (int d = 0; d < 4; ++d) {
+      if (d == pi) off[d] = GL4 * ((q & 1) ? 1.0 : -1.0);
+      if (d == pk) off[d] = GL4 * ((q & 2) ? 1.0 : -1.0);
+    }
     return;
   }
   const int m = p - 41;
   for (int i = 0; i < 4; ++i) off[i] = GL5 * (((m >> i) & 1) ? 1.0 : -1.0);
 }
-__device__ inline double gm_w7(int p) {
-  const double n = 4.0;
-  if (p == 0) return (12824.0 - 9120.0 * n + 400.0 * n * n) / 19683.0;
-  if (p <= 16) return ((p - 1) % 4 < 2) ? 980.0 / 6561.0 : (1820.0 - 400.0 * n) / 19683.0;
-  if (p <= 40) return 200.0 / 19683.0;
-  return 6859.0 / 19683.0 / 16.0;
-}
-__device__ inline double gm_w5(int p) {
-  const double n = 4.0;
-  if (p == 0) return (729.0 - 950.0 * n + 50.0 * n * n) / 729.0;
-  if (p <= 16) return ((p - 1) % 4 < 2) ? 245.0 / 486.0 : (265.0 - 100.0 * n) / 1458.0;
-  if (p <= 40) return 25.0 / 729.0;
-  return 0.0;
+// weights of the five classes of points (0: centre, 1: l2, 2: l4, 3: two
+// axes, 4: all axes) for four dimensions
+__device__ constexpr double kW7[5] = {(12824.0 - 9120.0 * 4 + 400.0 * 16) / 19683.0, 980.0 / 6561.0,
+                                      (1820.0 - 400.0 * 4) / 19683.0, 200.0 / 19683.0, 6859.0 / 19683.0 / 16.0};
+__device__ constexpr double kW5[5] = {(729.0 - 950.0 * 4 + 50.0 * 16) / 729.0, 245.0 / 486.0,
+                                      (265.0 - 100.0 * 4) / 1458.0, 25.0 / 729.0, 0.0};
+__device__ inline int gm_class(int p) { return p == 0 ? 0 : p <= 16 ? ((p - 1) % 4 < 2 ? 1 : 2) : p <= 40 ? 3 : 4; }
+
+__device__ __forceinline__ bool cub_done(const double te[2], const double tv[2]) {
+  for (int j = 0; j < 2; ++j)
+    if (te[j] > CUB_ABSTOL && te[j] > fabs(tv[j]) * CUB_RELTOL) return false;
+  return true;
 }
 
-// Evaluate the rule on nreg (1 or 2) regions with the whole warp.
-__device__ void gm_eval(const PairGeo& G, int ft, int fs, const double sep[3], Region* R, int nreg,
-                        double (*fv)[57][2]) {
+// A region of the adaptive cubature and the axis to split; its key, the larger
+// error, is kept in an array of its own, which the search for the largest runs
+// over.
+struct Region {
+  double c[4], h[4], val[2], err[2];
+  int split;
+};
+__device__ inline double region_key(const Region& r) { return r.err[0] > r.err[1] ? r.err[0] : r.err[1]; }
+
+__device__ inline double warp_add(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// One lane's share of the rule on a half-warp: four points, the l2 / l4
+// points 1 .. 16 first, then 17 .. 56 and the centre.
+struct GmLane {
+  double off[4][4], w7[4], w5[4];
+};
+__device__ inline void gm_lane(int li, GmLane& g) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = 16 * q + li, p = k < 56 ? k + 1 : 0, c = gm_class(p);
+    const bool on = k <= 56;
+    gm_point(p, g.off[q]);
+    g.w7[q] = on ? (c == 0 ? kW7[0] : c == 1 ? kW7[1] : c == 2 ? kW7[2] : c == 3 ? kW7[3] : kW7[4]) : 0.0;
+    g.w5[q] = on ? (c == 0 ? kW5[0] : c == 1 ? kW5[1] : c == 2 ? kW5[2] : c == 3 ? kW5[3] : kW5[4]) : 0.0;
+  }
+}
+__device__ __forceinline__ double half_add(double v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Genz-Malik rule on two regions by one warp, one per half-warp (Q: this
+// half's, c and h set); every lane ends with its half's val, err and split.
+template <bool RF>
+__device__ __forceinline__ void gm_eval(const PairLine& L, Z f, RealF rq, const GmLane& g, Region& Q) {
+  Z fv[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    double r2 = 0;
+    double u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = Q.c[i] + g.off[q][i] * Q.h[i];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double v = L.o[d] + (u[0] * L.a[0][d] + u[1] * L.a[1][d]) + (u[2] * L.a[2][d] + u[3] * L.a[3][d]);
+      r2 += v * v;
+    }
+    fv[q] = ego_at<RF>(r2, f, rq);
+  }
+  const double vol = (2.0 * Q.h[0]) * (2.0 * Q.h[1]) * ((2.0 * Q.h[2]) * (2.0 * Q.h[3]));
+  const double ratio = (GL2 * GL2) / (GL4 * GL4);
+  double dd = 0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    double s7 = 0, s5 = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double a = j ? fv[q].y : fv[q].x;
+      s7 = g.w7[q] != 0.0 ? fma(g.w7[q], a, s7) : s7;  // the idle share's value may be infinite
+      s5 = g.w5[q] != 0.0 ? fma(g.w5[q], a, s5) : s5;
+    }
+    s7 = half_add(s7);
+    s5 = half_add(s5);
+    Q.val[j] = vol * s7;
+    Q.err[j] = fabs(vol * s5 - vol * s7);
+    // fourth difference of axis i on lane 4 i (points -l2, +l2, -l4, +l4)
+    const double a = j ? fv[0].y : fv[0].x, z = j ? fv[3].y : fv[3].x;
+    const double f0 = __shfl_sync(0xffffffffu, z, 8, 16);
+    const double fb = __shfl_down_sync(0xffffffffu, a, 1), fc = __shfl_down_sync(0xffffffffu, a, 2),
+                 fd = __shfl_down_sync(0xffffffffu, a, 3);
+    dd += fabs(a + fb - 2 * f0 - ratio * (fc + fd - 2 * f0));
+  }
+  int sd = 0;
+  double md = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double d = __shfl_sync(0xffffffffu, dd, 4 * i, 16);
+    if (d > md) {
+      md = d;
+      sd = i;
+    }
+  }
+  Q.split = sd;
+}
+
+// hcubature(2, f, 0, 1; reltol, abstol, INDIVIDUAL) with the warp, its regions
+// in H and their keys in K (capacity cap): 1 done (out set on every lane), 0 the
+// capacity is exceeded.  The region of the largest error is split; the search
+// over the keys is a warp reduction (ties: the older region).
+template <bool RF>
+__device__ int cubature(const PairLine& L, Z f, RealF rq, const GmLane& g, Region* H, double* K, int cap,
+                        double out[2]) {
   const int lane = threadIdx.x & 31;
-  for (int p = lane; p < 57 * nreg; p += 32) {
-    const int r = p / 57, pp = p - r * 57;
-    double off[4], u[4];
-    gm_point(pp, off);
-    for (int i = 0; i < 4; ++i) u[i] = R[r].c[i] + off[i] * R[r].h[i];
-    face_val(G, ft, fs, sep, u, fv[r][pp]);
+  const bool up = lane >= 16;  // the half that takes the upper child
+  Region R;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) R.c[i] = R.h[i] = 0.5;
+  gm_eval<RF>(L, f, rq, g, R);
+  double tv[2] = {R.val[0], R.val[1]}, te[2] = {R.err[0], R.err[1]};
+  if (cub_done(te, tv)) {
+    out[0] = tv[0];
+    out[1] = tv[1];
+    return 1;
+  }
+  if (lane == 0) {
+    H[0] = R;
+    K[0] = region_key(R);
   }
   __syncwarp();
-  if (lane < nreg) {
-    Region& Q = R[lane];
-    const double ratio = (GL2 * GL2) / (GL4 * GL4);
-    double s7[2] = {0, 0}, s5[2] = {0, 0};
-    for (int p = 0; p < 57; ++p) {
-      const double a = gm_w7(p), b = gm_w5(p);
-      s7[0] += a * fv[lane][p][0];
-      s7[1] += a * fv[lane][p][1];
-      s5[0] += b * fv[lane][p][0];
-      s5[1] += b * fv[lane][p][1];
-    }
-    double vol = 1.0;
-    for (int i = 0; i < 4; ++i) vol *= 2.0 * Q.h[i];
-    Q.errmax = 0;
-    for (int j = 0; j < 2; ++j) {
-      Q.val[j] = vol * s7[j];
-      Q.err[j] = fabs(vol * s5[j] - vol * s7[j]);
-      if (Q.err[j] > Q.errmax) Q.errmax = Q.err[j];
-    }
-    int sd = 0;
-    double md = 0;
-    for (int i = 0; i < 4; ++i) {
-      double d = 0;
-      const double* f0 = fv[lane][0];
-      for (int j = 0; j < 2; ++j) {
-        const double fa = fv[lane][1 + 4 * i][j], fb = fv[lane][2 + 4 * i][j];
-        const double fc = fv[lane][3 + 4 * i][j], fd = fv[lane][4 + 4 * i][j];
-        d += fabs(fa + fb - 2 * f0[j] - ratio * (fc + fd - 2 * f0[j]));
-      }
-      if (d > md) {
-        md = d;
-        sd = i;
-      }
-    }
-    Q.split = sd;
-  }
-  __syncwarp();
-}
-
-// heap in global memory (lane 0 only)
-__device__ void hp_push(Region* H, int& nh, const Region& r) {
-  int i = nh++;
-  H[i] = r;
-  while (i > 0) {
-    const int p = (i - 1) / 2;
-    if (H[p].errmax >= H[i].errmax) break;
-    const Region t = H[p];
-    H[p] = H[i];
-    H[i] = t;
-    i = p;
-  }
-}
-__device__ Region hp_pop(Region* H, int& nh) {
-  const Region top = H[0];
-  H[0] = H[--nh];
-  int i = 0;
+  int n = 1;
   for (;;) {
-    const int l = 2 * i + 1, r = l + 1;
-    int m = i;
-    if (l < nh && H[l].errmax > H[m].errmax) m = l;
-    if (r < nh && H[r].errmax > H[m].errmax) m = r;
-    if (m == i) break;
-    const Region t = H[m];
-    H[m] = H[i];
-    H[i] = t;
-    i = m;
-  }
-  return top;
-}
-
-// hcubature(2, f, 0, 1; reltol, abstol, INDIVIDUAL) with the warp; returns
-// false (and sets *err) when the heap capacity or iteration cap is exceeded.
-__device__ bool cubature(const PairGeo& G, int ft, int fs, const double sep[3], Region* heap, int cap,
-                         Region* reg2, double (*fv)[57][2], double out[2], int* errflag) {
-  const int lane = threadIdx.x & 31;
-  if (lane == 0) {
-    for (int i = 0; i < 4; ++i) {
-      reg2[0].c[i] = 0.5;
-      reg2[0].h[i] = 0.5;
+    if (n + 1 > cap) return 0;
+    double bk = -1.0;
+    int bi = 0x7fffffff;
+    for (int i = lane; i < n; i += 32) {
+      const double k = K[i];
+      if (k > bk) {
+        bk = k;
+        bi = i;
+      }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double k = __shfl_xor_sync(0xffffffffu, bk, o);
+      const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (k > bk || (k == bk && i < bi)) {
+        bk = k;
+        bi = i;
+      }
+    }
+    if (bi >= n) bi = 0;  // every key NaN
+    R = H[bi];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      tv[j] -= R.val[j];
+      te[j] -= R.err[j];
+    }
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const double h = d == R.split ? R.h[d] * 0.5 : R.h[d];
+      R.c[d] = d == R.split ? (up ? R.c[d] + h : R.c[d] - h) : R.c[d];
+      R.h[d] = h;
+    }
+    gm_eval<RF>(L, f, rq, g, R);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      tv[j] += R.val[j] + __shfl_xor_sync(0xffffffffu, R.val[j], 16);
+      te[j] += R.err[j] + __shfl_xor_sync(0xffffffffu, R.err[j], 16);
+    }
+    __syncwarp();
+    if ((lane & 15) == 0) {
+      const int at = up ? n : bi;
+      H[at] = R;
+      K[at] = region_key(R);
+    }
+    ++n;
+    __syncwarp();
+    if (cub_done(te, tv)) break;
   }
+  double s0 = 0, s1 = 0;
+  for (int i = lane; i < n; i += 32) {
+    s0 += H[i].val[0];
+    s1 += H[i].val[1];
+  }
+  out[0] = warp_add(s0);
+  out[1] = warp_add(s1);
   __syncwarp();
-  gm_eval(G, ft, fs, sep, reg2, 1, fv);
-  __shared__ int s_done[8];
-  const int wid = threadIdx.x >> 5;
-  double tv[2] = {reg2[0].val[0], reg2[0].val[1]}, te[2] = {reg2[0].err[0], reg2[0].err[1]};
-  int nh = 0;
-  if (lane == 0) hp_push(heap, nh, reg2[0]);
-  bool ok = true;
-  for (int it = 0;; ++it) {
-    if (lane == 0) {
-      int conv = 1;
-      for (int j = 0; j < 2; ++j)
-        if (te[j] > CUB_ABSTOL && te[j] > fabs(tv[j]) * CUB_RELTOL) conv = 0;
-      int stop = conv;
-      if (!conv && (nh + 2 > cap || it > 4000000)) {
-        if (errflag) atomicOr(errflag, 1);  // else the caller defers the item
-        stop = 2;
-      }
-      if (!stop) {
-        const Region R = hp_pop(heap, nh);
-        for (int j = 0; j < 2; ++j) {
-          tv[j] -= R.val[j];
-          te[j] -= R.err[j];
-        }
-        reg2[0] = R;
-        reg2[1] = R;
-        const int d = R.split;
-        reg2[0].h[d] = reg2[1].h[d] = R.h[d] * 0.5;
-        reg2[0].c[d] = R.c[d] - reg2[0].h[d];
-        reg2[1].c[d] = R.c[d] + reg2[0].h[d];
-      }
-      s_done[wid] = stop;
-    }
-    __syncwarp();
-    const int stop = s_done[wid];
-    __syncwarp();
-    if (stop) {
-      ok = stop == 1;
-      break;
-    }
-    gm_eval(G, ft, fs, sep, reg2, 2, fv);
-    if (lane == 0) {
-      for (int j = 0; j < 2; ++j) {
-        tv[j] += reg2[0].val[j] + reg2[1].val[j];
-        te[j] += reg2[0].err[j] + reg2[1].err[j];
-      }
-      hp_push(heap, nh, reg2[0]);
-      hp_push(heap, nh, reg2[1]);
-    }
-    __syncwarp();
-  }
-  if (lane == 0) {
-    out[0] = out[1] = 0;
-    for (int i = 0; i < nh; ++i) {
-      out[0] += heap[i].val[0];
-      out[1] += heap[i].val[1];
-    }
-  }
-  __syncwarp();
-  return ok;
+  return 1;
 }
 
 // srfSum! restricted to the six stored components, accumulated in the
@@ -764,101 +943,223 @@ __device__ inline void srf_sum6(const Z* s_, Z out[6]) {
   out[5] = zsub(zadd(zadd(Z{-s[17].x, -s[17].y}, s[18]), s[23]), s[24]);
 }
 
-// Far offsets: warp per offset, persistent over a work counter.
+// Far offsets of a chunk of items [item0, item0 + n):
 //   mode 0 (self):  offset (ix,iy,iz) of the Toeplitz field, skipped when all
 //                   indices <= 1 (near); sep = index * pitch;
 //   mode 1 (ext):   circulant index; split indices zero; touching offsets are
 //                   left to the contact kernel; sep from the grdSel tables.
+// Three steps: k_far_first evaluates the rule once on the whole domain of
+// every face pair (nearly all pairs of separated cells converge there) and
+// lists the others; k_adapt refines the listed ones; k_far_sum combines the
+// records of the items that had any.
 struct FarParams {
   int mode;
   int n[3];                 // extents of the output field
-  int64_t nitems;
   const double* sep[3];     // per-axis separation tables
   int split[3];             // ext: 0-based split index (trg cel), self: -1
   double touch[3];          // ext contact threshold per axis (cntTol + (sT+sS)/2), or -1
   Z* out;                   // [6][n2][n1][n0]
-  Region* heap;             // per-warp heaps
-  int cap;
-  unsigned long long* counter;
-  int* errflag;
-  // overflow handling: the first pass (list == nullptr) appends items whose
-  // region heap overflowed to ovf_list and leaves them to a second pass over
-  // that list with larger heaps (list != nullptr, *list_count items)
-  const int64_t* list;
-  const unsigned long long* list_count;
-  int64_t* ovf_list;
-  unsigned long long* ovf_count;
+};
+// a face pair to refine: its 24 values' record and place in it
+struct Unit {
+  int rec, pair;
+};
+// an item with listed pairs: the output element (near and far offsets of one
+// field) and its separation
+struct Rec {
+  int64_t o;
+  double sep[3];
+};
+// Work lists of one build: counters [0] records, [1] units, [2] next unit of
+// k_adapt's first pass, [3] deferred units, [4] next deferred unit, [5], [6]
+// the same for the last pass.
+struct Lists {
+  Rec* rec;
+  Z* val;      // [rec][24] scaled pair values
+  Unit* unit;
+  Unit* ovf[2];
+  int* cnt;
 };
 
-__global__ void __launch_bounds__(128) k_far(const FarParams p, const PairGeo* __restrict__ gp) {
-  __shared__ PairGeo G;
-  __shared__ Region reg2s[4][2];
-  __shared__ double fvs[4][2][57][2];
-  __shared__ Z srf[4][36];
-  __shared__ unsigned long long s_item[4];
-  for (int i = threadIdx.x; i < (int)(sizeof(PairGeo) / sizeof(double)); i += blockDim.x)
-    reinterpret_cast<double*>(&G)[i] = reinterpret_cast<const double*>(gp)[i];
-  __syncthreads();
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
-  Region* heap = p.heap + gw * p.cap;
+// Items one block takes at a time.  A thread runs the 57 points of one
+// (item, pair) by itself -- no reductions, and the pairs of a warp differ only
+// in the table column and the separation they read.  Bound by FP64 arithmetic:
+// the warp-per-offset form before it spent its time in the serial sums and
+// the global-memory heap of its one active lane (32^3 cells: 9.0 ms, now 0.26
+// ms and 0.13 ms of k_adapt).
+constexpr int kFarItems = 32;
+template <bool RF>
+__global__ void __launch_bounds__(256) k_far_first(const FarParams p, const PairGeo* __restrict__ gp, int64_t item0,
+                                                   int64_t nitems, const Lists L) {
+  __shared__ double D[3][kGm][24];  // face-to-face vectors of the points at separation 0
+  __shared__ Z srf[kFarItems][24];
+  __shared__ double sepi[kFarItems][3];
+  __shared__ double scale[24];
+  __shared__ int rec[kFarItems], state[kFarItems];  // 0 evaluate, 1 nothing to do
+  __shared__ unsigned open[kFarItems];              // pairs that need refining
+  for (int q = threadIdx.x; q < kGm * 24; q += blockDim.x) {
+    const int pt = q / 24, k = q % 24;
+    double off[4];
+    gm_point(pt, off);
+    const double zero[3] = {0, 0, 0};
+    const PairLine l = pair_line(*gp, c_pairs[k], zero);
+    for (int d = 0; d < 3; ++d) {
+      double v = l.o[d];
+      for (int i = 0; i < 4; ++i) v += (0.5 + off[i] * 0.5) * l.a[i][d];
+      D[d][pt][k] = v;
+    }
+  }
+  if (threadIdx.x < 24) scale[threadIdx.x] = gp->scale[c_pairs[threadIdx.x]];
+  const Z f = gp->f;
+  const RealF rq{f.x, 1.0 / (4.0 * PI * f.x * f.x)};
   const int64_t plane = (int64_t)p.n[0] * p.n[1], vol = plane * p.n[2];
-  const int64_t nitems = p.list ? (int64_t)*p.list_count : p.nitems;
-  for (;;) {
-    if (lane == 0) s_item[wid] = atomicAdd(p.counter, 1ull);
-    __syncwarp();
-    const unsigned long long ticket = s_item[wid];
-    __syncwarp();
-    if ((int64_t)ticket >= nitems) break;
-    const unsigned long long item = p.list ? (unsigned long long)p.list[ticket] : ticket;
-    const int ix = (int)(item % p.n[0]), iy = (int)((item / p.n[0]) % p.n[1]), iz = (int)(item / plane);
-    const int id[3] = {ix, iy, iz};
-    bool skip = false, zero = false;
-    double sep[3];
-    for (int d = 0; d < 3; ++d) sep[d] = p.sep[d][id[d]];
-    if (p.mode == 0) {
-      skip = !(ix > 1 || iy > 1 || iz > 1);
-    } else {
-      for (int d = 0; d < 3; ++d) zero |= id[d] == p.split[d];
-      if (!zero && p.touch[0] > 0) {
-        bool t = true;
-        for (int d = 0; d < 3; ++d) t &= fabs(sep[d]) < p.touch[d];
-        skip = t;
+  for (int64_t b0 = (int64_t)blockIdx.x * kFarItems; b0 < nitems; b0 += (int64_t)gridDim.x * kFarItems) {
+    __syncthreads();
+    if (threadIdx.x < kFarItems) {
+      const int64_t item = item0 + b0 + threadIdx.x;
+      int st = 1;
+      if (b0 + threadIdx.x < nitems) {
+        const int id[3] = {(int)(item % p.n[0]), (int)((item / p.n[0]) % p.n[1]), (int)(item / plane)};
+        bool skip = false, zero = false;
+        double sep[3];
+        for (int d = 0; d < 3; ++d) sepi[threadIdx.x][d] = sep[d] = p.sep[d][id[d]];
+        if (p.mode == 0) {
+          skip = !(id[0] > 1 || id[1] > 1 || id[2] > 1);
+        } else {
+          for (int d = 0; d < 3; ++d) zero |= id[d] == p.split[d];
+          if (!zero && p.touch[0] > 0) {
+            bool t = true;
+            for (int d = 0; d < 3; ++d) t &= fabs(sep[d]) < p.touch[d];
+            skip = t;
+          }
+        }
+        if (!skip && zero)
+          for (int c = 0; c < 6; ++c) p.out[c * vol + item] = Z{0, 0};
+        st = skip || zero;
+      }
+      state[threadIdx.x] = st;
+      open[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    for (int u = threadIdx.x; u < kFarItems * 24; u += blockDim.x) {
+      const int it = u / 24, k = u % 24;
+      if (state[it]) continue;
+      const double sx = sepi[it][0], sy = sepi[it][1], sz = sepi[it][2];
+      auto at = [&](int pt) -> Z {
+        const double x = D[0][pt][k] + sx, y = D[1][pt][k] + sy, z = D[2][pt][k] + sz;
+        return ego_at<RF>(x * x + y * y + z * z, f, rq);
+      };
+      const Z s0 = at(0);
+      Z s1{0, 0}, s2{0, 0}, s3{0, 0}, s4{0, 0};
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        s1 = zadd(s1, zadd(at(1 + 4 * i), at(2 + 4 * i)));
+        s2 = zadd(s2, zadd(at(3 + 4 * i), at(4 + 4 * i)));
+      }
+#pragma unroll 2
+      for (int pt = 17; pt <= 40; ++pt) s3 = zadd(s3, at(pt));
+#pragma unroll 2
+      for (int pt = 41; pt < kGm; ++pt) s4 = zadd(s4, at(pt));
+      auto sum = [&](const double* w) -> Z {
+        return Z{w[0] * s0.x + w[1] * s1.x + w[2] * s2.x + w[3] * s3.x + w[4] * s4.x,
+                 w[0] * s0.y + w[1] * s1.y + w[2] * s2.y + w[3] * s3.y + w[4] * s4.y};
+      };
+      const Z v7 = sum(kW7), v5 = sum(kW5);
+      const double tv[2] = {v7.x, v7.y}, te[2] = {fabs(v5.x - v7.x), fabs(v5.y - v7.y)};
+      srf[it][k] = zsc(v7, scale[k]);
+      if (!cub_done(te, tv)) atomicOr(&open[it], 1u << k);
+    }
+    __syncthreads();
+    if (threadIdx.x < kFarItems && !state[threadIdx.x]) {
+      const int it = threadIdx.x;
+      const int64_t o = item0 + b0 + it;
+      if (open[it]) {
+        const int r = atomicAdd(L.cnt, 1);
+        rec[it] = r;
+        L.rec[r] = Rec{o, {sepi[it][0], sepi[it][1], sepi[it][2]}};
+        int u = atomicAdd(L.cnt + 1, __popc(open[it]));
+        for (int k = 0; k < 24; ++k)
+          if (open[it] >> k & 1) L.unit[u++] = Unit{r, k};
+      } else {
+        Z s[36], c6[6];
+        for (int k = 0; k < 36; ++k) s[k] = Z{0, 0};
+        for (int k = 0; k < 24; ++k) s[kPairs[k]] = srf[it][k];
+        srf_sum6(s, c6);
+        for (int c = 0; c < 6; ++c) p.out[c * vol + o] = c6[c];
       }
     }
-    if (skip) continue;
-    const int64_t o = ((int64_t)iz * p.n[1] + iy) * p.n[0] + ix;
-    if (zero) {
-      if (lane < 6) p.out[lane * vol + o] = Z{0, 0};
-      continue;
+    __syncthreads();
+    for (int u = threadIdx.x; u < kFarItems * 24; u += blockDim.x) {
+      const int it = u / 24, k = u % 24;
+      if (!state[it] && open[it] && !(open[it] >> k & 1)) L.val[(int64_t)rec[it] * 24 + k] = srf[it][k];
     }
-    for (int k = lane; k < 36; k += 32) srf[wid][k] = Z{0, 0};
-    __syncwarp();
-    bool ok = true;
-    for (int k = 0; k < 24 && ok; ++k) {
-      const int fp = c_pairs[k];
-      double v[2];
-      ok = cubature(G, fp / 6, fp % 6, sep, heap, p.cap, reg2s[wid], fvs[wid], v, p.ovf_list ? nullptr : p.errflag);
-      if (lane == 0) srf[wid][fp] = zsc(Z{v[0], v[1]}, G.scale[fp]);
-      __syncwarp();
-    }
-    if (!ok) {
-      if (lane == 0 && p.ovf_list) p.ovf_list[atomicAdd(p.ovf_count, 1ull)] = (int64_t)item;
-      __syncwarp();
-      continue;
-    }
+  }
+}
+
+// The listed face pairs, one warp each, over a work counter.  pass 0: regions
+// in shared memory (kCap0 each, four warps a block); a pair that needs more
+// goes to the next list.  pass 1: that list, kCap1 regions in shared memory,
+// one warp a block; pass 2: kCap2 in global memory, past which the build
+// fails.  A pair is a chain of dependent rule evaluations, so its latency
+// counts (near pairs of a cubic cell: 0.81 ms with pass 1's regions in global
+// memory and the two child regions one after the other, 0.53 ms with a
+// half-warp each; 15.3 ms with all 36 pairs of an offset on one warp).
+constexpr int kCap0 = 48, kCap1 = 512, kCap2 = 16384;
+constexpr int kRegBytes = sizeof(Region) + sizeof(double);
+template <bool RF>
+__global__ void k_adapt(const PairGeo* __restrict__ gp, const Lists L, int pass, unsigned char* heap, int cap,
+                        int* errflag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  unsigned char* const own = heap ? heap + (size_t)(blockIdx.x * nw + wid) * cap * kRegBytes
+                                  : smem_raw + (size_t)wid * cap * kRegBytes;
+  Region* const H = reinterpret_cast<Region*>(own);
+  double* const K = reinterpret_cast<double*>(H + cap);
+  const Unit* const list = pass == 0 ? L.unit : L.ovf[pass - 1];
+  const int n = L.cnt[1 + 2 * pass];
+  const Z f = gp->f;
+  const RealF rq{f.x, 1.0 / (4.0 * PI * f.x * f.x)};
+  GmLane g;
+  gm_lane(lane & 15, g);
+  for (;;) {
+    int k = 0;
+    if (lane == 0) k = atomicAdd(L.cnt + 2 + 2 * pass, 1);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= n) break;
+    const Unit u = list[k];
+    const int fp = c_pairs[u.pair];
+    const PairLine pl = pair_line(*gp, fp, L.rec[u.rec].sep);
+    double v[2];
+    const int ok = cubature<RF>(pl, f, rq, g, H, K, cap, v);
     if (lane == 0) {
-      Z c6[6];
-      srf_sum6(srf[wid], c6);
-      for (int c = 0; c < 6; ++c) p.out[c * vol + o] = c6[c];
+      if (ok)
+        L.val[(int64_t)u.rec * 24 + u.pair] = zsc(Z{v[0], v[1]}, gp->scale[fp]);
+      else if (pass < 2)
+        L.ovf[pass][atomicAdd(L.cnt + 3 + 2 * pass, 1)] = u;
+      else
+        atomicOr(errflag, 1);
     }
     __syncwarp();
   }
 }
 
-// Near offsets of a self operator (egoFunSng!, src/glaGen.jl:350-528): one
-// warp per offset (px, py, pz) in {0,1}^3 within the volume; corrected pairs
-// from the weak values, the others by cubature.
+// the six components of every record
+__global__ void k_far_sum(const FarParams p, const Lists L) {
+  const int n = L.cnt[0];
+  const int64_t vol = (int64_t)p.n[0] * p.n[1] * p.n[2];
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    Z s[36], c6[6];
+    for (int k = 0; k < 36; ++k) s[k] = Z{0, 0};
+    for (int k = 0; k < 24; ++k) s[kPairs[k]] = L.val[(int64_t)r * 24 + k];
+    srf_sum6(s, c6);
+    for (int c = 0; c < 6; ++c) p.out[c * vol + L.rec[r].o] = c6[c];
+  }
+}
+
+// Near offsets of a self operator (egoFunSng!, src/glaGen.jl:350-528): offsets
+// (px, py, pz) in {0,1}^3 within the volume, one block each; the corrected
+// pairs from the weak values, the others listed for k_adapt.  Pairs that feed
+// none of the six components are not evaluated.
 __constant__ signed char c_sng_cor[8][6][6];
 __constant__ signed char c_sng_mask[8][6][6];
 
@@ -867,51 +1168,29 @@ struct NearParams {
   int cases[8];  // egoFunSng! case per offset (x fastest), -1 = every pair by cubature
   const double* sep[3];
   const Z* weak;  // 18 scaled weak values
-  Z* out;         // toe [6][...]
-  Region* heap;
-  int cap;
-  int* errflag;
 };
 
-__global__ void __launch_bounds__(32) k_near(const NearParams p, const PairGeo* __restrict__ gp) {
-  __shared__ PairGeo G;
-  __shared__ Region reg2[2];
-  __shared__ double fv[2][57][2];
-  __shared__ Z srf[36];
-  for (int i = threadIdx.x; i < (int)(sizeof(PairGeo) / sizeof(double)); i += blockDim.x)
-    reinterpret_cast<double*>(&G)[i] = reinterpret_cast<const double*>(gp)[i];
-  __syncthreads();
+__global__ void __launch_bounds__(32) k_near_list(const NearParams p, const Lists L) {
+  __shared__ int rec;
   const int b = blockIdx.x;
   const int px = b & 1, py = (b >> 1) & 1, pz = (b >> 2) & 1;
   if (px >= p.n[0] || py >= p.n[1] || pz >= p.n[2]) return;
-  const int cs = p.cases[b];
-  const int lane = threadIdx.x;
-  Region* heap = p.heap + (int64_t)b * p.cap;
-  const double sep[3] = {p.sep[0][px], p.sep[1][py], p.sep[2][pz]};
-  for (int k = lane; k < 36; k += 32) srf[k] = Z{0, 0};
-  __syncwarp();
-  for (int fp = 0; fp < 36; ++fp) {
-    const int a = fp / 6, c = fp % 6;
-    const int m = cs < 0 ? 0 : c_sng_mask[cs][a][c];
-    if (m) {
-      if (lane == 0) {
-        const int code = c_sng_cor[cs][a][c];
-        srf[fp] = code == 0 ? Z{0, 0} : code < 10 ? p.weak[code - 1] : code < 20 ? p.weak[3 + code - 11]
-                                                                                  : p.weak[12 + code - 21];
-      }
-    } else {
-      double v[2];
-      cubature(G, a, c, sep, heap, p.cap, reg2, fv, v, p.errflag);
-      if (lane == 0) srf[fp] = zsc(Z{v[0], v[1]}, G.scale[fp]);
-    }
-    __syncwarp();
+  if (threadIdx.x == 0) {
+    rec = atomicAdd(L.cnt, 1);
+    L.rec[rec] = Rec{((int64_t)pz * p.n[1] + py) * p.n[0] + px, {p.sep[0][px], p.sep[1][py], p.sep[2][pz]}};
   }
-  if (lane == 0) {
-    Z c6[6];
-    srf_sum6(srf, c6);
-    const int64_t vol = (int64_t)p.n[0] * p.n[1] * p.n[2];
-    const int64_t o = ((int64_t)pz * p.n[1] + py) * p.n[0] + px;
-    for (int c = 0; c < 6; ++c) p.out[c * vol + o] = c6[c];
+  __syncwarp();
+  const int k = threadIdx.x, cs = p.cases[b];
+  if (k >= 24) return;
+  const int a = c_pairs[k] / 6, c = c_pairs[k] % 6;
+  if (cs >= 0 && c_sng_mask[cs][a][c]) {
+    const int code = c_sng_cor[cs][a][c];
+    L.val[(int64_t)rec * 24 + k] = code == 0   ? Z{0, 0}
+                                   : code < 10 ? p.weak[code - 1]
+                                   : code < 20 ? p.weak[3 + code - 11]
+                                               : p.weak[12 + code - 21];
+  } else {
+    L.unit[atomicAdd(L.cnt + 1, 1)] = Unit{rec, k};
   }
 }
 
@@ -1335,86 +1614,134 @@ struct Build {
   }
 };
 
+// the fast kernel values' condition (ego_line)
+static bool real_freq(Z f) { return f.y == 0.0 && f.x != 0.0; }
+
 // weak values (18, scaled by 1/prod(scl)) for a cell of size scl; the
 // unscaled values go to raw_out when given
 static gila_status weak_values(Build& B, const Rat sclr[3], Z* w_d, Z* raw_out = nullptr) {
   const double scl[3] = {rd(sclr[0]), rd(sclr[1]), rd(sclr[2])};
-  std::vector<WItem> items = weak_items(scl);
-  const int n = (int)items.size(), ord = B.ord;
+  const std::vector<WItem> all = weak_items(scl);
+  const int ord = B.ord;
+  // items that repeat another's type and vertices (cells with equal sides)
+  // are evaluated once; grouped by kind
+  std::vector<WItem> items;
+  std::vector<int> uid(all.size());
+  int first[4] = {0, 0, 0, 0};
+  for (int kind = 0; kind < 3; ++kind) {
+    for (size_t i = 0; i < all.size(); ++i) {
+      const int t = all[i].type;
+      if ((t == W_S ? 0 : t == W_E ? 1 : 2) != kind) continue;
+      size_t k = 0;
+      while (k < items.size() && (items[k].type != t || memcmp(&items[k].t, &all[i].t, sizeof(Tri6)) != 0)) ++k;
+      uid[i] = (int)k;
+      if (k == items.size()) items.push_back(all[i]);
+    }
+    first[kind + 1] = (int)items.size();
+  }
+  const int n = (int)items.size();
   WItem* it_d;
   gila_status s;
   if ((s = B.alloc(&it_d, items.size())) != GILA_OK) return s;
   KB_TRY(cudaMemcpyAsync(it_d, items.data(), items.size() * sizeof(WItem), cudaMemcpyHostToDevice, B.st));
   const int max_outer = 24 * ord;
   Z *part_d, *sums_d, *raw_d;
-  int* nout_d;
+  int* uid_d;
   if ((s = B.alloc(&part_d, (size_t)n * max_outer)) != GILA_OK) return s;
   if ((s = B.alloc(&sums_d, n)) != GILA_OK) return s;
   if (raw_out)
     raw_d = raw_out;
   else if ((s = B.alloc(&raw_d, 18)) != GILA_OK)
     return s;
-  if ((s = B.alloc(&nout_d, n)) != GILA_OK) return s;
-  std::vector<int> nout(n);
-  for (int i = 0; i < n; ++i) {
-    const int t = items[i].type;
-    nout[i] = t == W_S ? 24 * ord : t == W_E ? 6 * ord : ord;
+  if ((s = B.alloc(&uid_d, uid.size())) != GILA_OK) return s;
+  KB_TRY(cudaMemcpyAsync(uid_d, uid.data(), uid.size() * sizeof(int), cudaMemcpyHostToDevice, B.st));
+  auto weak = [&](auto kern, int kind, int outer) {
+    const int m = first[kind + 1] - first[kind];
+    kern<<<m * outer, 256, 0, B.st>>>(it_d, first[kind], outer, max_outer, B.q_d, part_d);
+    return cudaGetLastError();
+  };
+  if (real_freq(B.f)) {
+    KB_TRY(weak(k_weak<2, true>, 2, ord));
+    KB_TRY(weak(k_weak<1, true>, 1, 6 * ord));
+    KB_TRY(weak(k_weak<0, true>, 0, 24 * ord));
+  } else {
+    KB_TRY(weak(k_weak<2, false>, 2, ord));
+    KB_TRY(weak(k_weak<1, false>, 1, 6 * ord));
+    KB_TRY(weak(k_weak<0, false>, 0, 24 * ord));
   }
-  KB_TRY(cudaMemcpyAsync(nout_d, nout.data(), n * sizeof(int), cudaMemcpyHostToDevice, B.st));
-  // one launch per item (grid = the item's outer sum); items are independent
-  for (int i = 0; i < n; ++i) {
-    k_weak<<<dim3(nout[i], 1), 256, 0, B.st>>>(it_d, i, max_outer, B.q_d, part_d);
-    KB_TRY(cudaGetLastError());
-  }
-  k_weak_reduce<<<(n + 127) / 128, 128, 0, B.st>>>(it_d, n, nout_d, part_d, max_outer, sums_d);
+  k_weak_reduce<<<n, 32, 0, B.st>>>(it_d, ord, part_d, max_outer, sums_d);
   KB_TRY(cudaGetLastError());
   double* scl_d;
   if ((s = B.alloc(&scl_d, 3)) != GILA_OK) return s;
   KB_TRY(cudaMemcpyAsync(scl_d, scl, sizeof(scl), cudaMemcpyHostToDevice, B.st));
   const double inv = rd(rdv(R(1), rmul(rmul(sclr[0], sclr[1]), sclr[2])));
-  k_weak_combine<<<1, 32, 0, B.st>>>(sums_d, scl_d, inv, B.f, w_d, raw_d);
+  k_weak_combine<<<1, 32, 0, B.st>>>(sums_d, uid_d, scl_d, inv, B.f, w_d, raw_d);
   KB_TRY(cudaGetLastError());
   return GILA_OK;
 }
 
-// Far pass over nitems with 512-region heaps, then the deferred items with
-// 16384-region heaps on 128 warps.
-static gila_status run_far(Build& B, FarParams fp, const PairGeo* g_d) {
+// The cubature's work lists, for chunks of at most kFarChunk items, and the
+// last pass's regions.
+constexpr int kFarChunk = 1 << 15, kWarps2 = 8;
+struct Cub {
+  Lists L;
+  unsigned char* heap;
+  const PairGeo* g;
+  int* err;
+};
+static gila_status cub_alloc(Build& B, int64_t nitems, const PairGeo* g_d, int* err_d, Cub* q) {
   gila_status s;
-  int nsm = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  int64_t blocks = (int64_t)nsm * 4;
-  const int64_t need = (fp.nitems + 3) / 4;
-  if (blocks > need) blocks = need < 1 ? 1 : need;
-  const int cap1 = 512, cap2 = 16384;
-  Region* heap;
-  if ((s = B.alloc(&heap, (size_t)blocks * 4 * cap1)) != GILA_OK) return s;
-  unsigned long long* cnt;
-  if ((s = B.alloc(&cnt, 3)) != GILA_OK) return s;
-  KB_TRY(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned long long), B.st));
-  int64_t* ovf;
-  if ((s = B.alloc(&ovf, (size_t)(fp.nitems > 0 ? fp.nitems : 1))) != GILA_OK) return s;
-  fp.heap = heap;
-  fp.cap = cap1;
-  fp.counter = cnt;
-  fp.list = nullptr;
-  fp.list_count = nullptr;
-  fp.ovf_list = ovf;
-  fp.ovf_count = cnt + 1;
-  k_far<<<(unsigned)blocks, 128, 0, B.st>>>(fp, g_d);
+  const size_t n = (size_t)std::min<int64_t>(std::max<int64_t>(nitems, 1), kFarChunk) + 8;
+  q->g = g_d;
+  q->err = err_d;
+  if ((s = B.alloc(&q->L.rec, n)) != GILA_OK) return s;
+  if ((s = B.alloc(&q->L.val, n * 24)) != GILA_OK) return s;
+  for (Unit** u : {&q->L.unit, &q->L.ovf[0], &q->L.ovf[1]})
+    if ((s = B.alloc(u, n * 24)) != GILA_OK) return s;
+  if ((s = B.alloc(&q->L.cnt, 8)) != GILA_OK) return s;
+  return B.alloc(&q->heap, (size_t)kWarps2 * kCap2 * kRegBytes);
+}
+static gila_status cub_reset(Build& B, Cub& q) {
+  KB_TRY(cudaMemsetAsync(q.L.cnt, 0, 8 * sizeof(int), B.st));
+  return GILA_OK;
+}
+// refines the listed pairs and writes the records' components
+static gila_status cub_finish(Build& B, Cub& q, const FarParams& fp) {
+  auto adapt = [&](int pass, int blocks, int threads, unsigned char* heap, int cap) -> cudaError_t {
+    const void* fn = real_freq(B.f) ? (const void*)k_adapt<true> : (const void*)k_adapt<false>;
+    const size_t sm = heap ? 0 : (size_t)threads / 32 * cap * kRegBytes;
+    if (sm > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (e != cudaSuccess) return e;
+    }
+    if (real_freq(B.f))
+      k_adapt<true><<<blocks, threads, sm, B.st>>>(q.g, q.L, pass, heap, cap, q.err);
+    else
+      k_adapt<false><<<blocks, threads, sm, B.st>>>(q.g, q.L, pass, heap, cap, q.err);
+    return cudaGetLastError();
+  };
+  KB_TRY(adapt(0, 592, 128, nullptr, kCap0));
+  KB_TRY(adapt(1, 592, 32, nullptr, kCap1));
+  KB_TRY(adapt(2, kWarps2 / 4, 128, q.heap, kCap2));
+  k_far_sum<<<148, 128, 0, B.st>>>(fp, q.L);
   KB_TRY(cudaGetLastError());
-  Region* heap2;
-  if ((s = B.alloc(&heap2, (size_t)32 * 4 * cap2)) != GILA_OK) return s;
-  fp.heap = heap2;
-  fp.cap = cap2;
-  fp.counter = cnt + 2;
-  fp.list = ovf;
-  fp.list_count = cnt + 1;
-  fp.ovf_list = nullptr;
-  fp.ovf_count = nullptr;
-  k_far<<<32, 128, 0, B.st>>>(fp, g_d);
-  KB_TRY(cudaGetLastError());
+  return GILA_OK;
+}
+// the far items of a field; units already listed (near offsets) are refined
+// with the first chunk
+static gila_status run_far(Build& B, Cub& q, const FarParams& fp, int64_t nitems) {
+  gila_status s;
+  for (int64_t i0 = 0; i0 < nitems; i0 += kFarChunk) {
+    const int64_t n = std::min<int64_t>(kFarChunk, nitems - i0);
+    const int64_t blocks = std::min<int64_t>(2 * 148, (n + kFarItems - 1) / kFarItems);
+    if (i0 > 0 && (s = cub_reset(B, q)) != GILA_OK) return s;
+    if (real_freq(B.f))
+      k_far_first<true><<<(unsigned)blocks, 256, 0, B.st>>>(fp, q.g, i0, n, q.L);
+    else
+      k_far_first<false><<<(unsigned)blocks, 256, 0, B.st>>>(fp, q.g, i0, n, q.L);
+    KB_TRY(cudaGetLastError());
+    if ((s = cub_finish(B, q, fp)) != GILA_OK) return s;
+  }
   return GILA_OK;
 }
 
@@ -1441,23 +1768,6 @@ static gila_status self_circulant(Build& B, const HVol& v, Z* crc_d, int* err_d)
     if ((s = B.alloc(&sep_d[d], sp.size())) != GILA_OK) return s;
     KB_TRY(cudaMemcpyAsync(sep_d[d], sp.data(), sp.size() * sizeof(double), cudaMemcpyHostToDevice, B.st));
   }
-  // near offsets
-  NearParams np;
-  for (int d = 0; d < 3; ++d) {
-    np.n[d] = (int)v.cel[d];
-    np.sep[d] = sep_d[d];
-  }
-  for (int b = 0; b < 8; ++b) np.cases[b] = sng_case((b & 1) + 1, ((b >> 1) & 1) + 1, ((b >> 2) & 1) + 1, v);
-  np.weak = w_d;
-  np.out = toe_d;
-  np.cap = 16384;
-  np.errflag = err_d;
-  Region* nheap;
-  if ((s = B.alloc(&nheap, (size_t)8 * np.cap)) != GILA_OK) return s;
-  np.heap = nheap;
-  k_near<<<8, 32, 0, B.st>>>(np, g_d);
-  KB_TRY(cudaGetLastError());
-  // far offsets
   FarParams fp{};
   fp.mode = 0;
   for (int d = 0; d < 3; ++d) {
@@ -1466,16 +1776,31 @@ static gila_status self_circulant(Build& B, const HVol& v, Z* crc_d, int* err_d)
     fp.split[d] = -1;
     fp.touch[d] = -1;
   }
-  fp.nitems = V;
   fp.out = toe_d;
-  fp.errflag = err_d;
-  if ((s = run_far(B, fp, g_d)) != GILA_OK) return s;
+  Cub cub;
+  if ((s = cub_alloc(B, V, g_d, err_d, &cub)) != GILA_OK) return s;
+  if ((s = cub_reset(B, cub)) != GILA_OK) return s;
+  // near offsets
+  NearParams np;
+  for (int d = 0; d < 3; ++d) {
+    np.n[d] = (int)v.cel[d];
+    np.sep[d] = sep_d[d];
+  }
+  for (int b = 0; b < 8; ++b) np.cases[b] = sng_case((b & 1) + 1, ((b >> 1) & 1) + 1, ((b >> 2) & 1) + 1, v);
+  np.weak = w_d;
+  k_near_list<<<8, 32, 0, B.st>>>(np, cub.L);
+  KB_TRY(cudaGetLastError());
+  // far offsets
+  if ((s = run_far(B, cub, fp, V)) != GILA_OK) return s;
   // identity + circulant embedding
   const Z id = zdiv(Z{1.0, 0.0}, zmul(B.f, B.f));
   k_embed<<<1184, 256, 0, B.st>>>(toe_d, (int)nx, (int)ny, (int)nz, id, crc_d);
   KB_TRY(cudaGetLastError());
   return GILA_OK;
 }
+
+// lengths with compile-time x and y passes
+static bool pass_length(int P) { return !ct_tiles(16, P, false).empty() || mx_ops<double2>(P); }
 
 // FP64 forward 3-D FFT of the 6-component circulant, in place
 static gila_status fft3(Build& B, Z* crc_d, const int P[3]) {
@@ -1484,6 +1809,29 @@ static gila_status fft3(Build& B, Z* crc_d, const int P[3]) {
   for (int ax = 0; ax < 3; ++ax) {
     AxisPlan pl;
     if ((s = plan_axis(P[ax], &pl)) != GILA_OK) return s;
+    if (pass_length(P[ax])) {
+      // the matvec's x and y passes on whole lines, in place: rows, or kx
+      // tiles of 6 Pz planes (y), or of 6 planes with a row of Px Py (z)
+      const void* tw;
+      if ((s = twiddle_table(B.ctx, P[ax], GILA_C128, &tw)) != GILA_OK) return s;
+      double2* const c = reinterpret_cast<double2*>(crc_d);
+      DevOp<double2> d{};
+      Geom g{};
+      const int k = ax == 0 ? 0 : 1;
+      d.plan[k] = pl;
+      d.tw[k] = static_cast<const double2*>(tw);
+      g.sc[k] = g.tc[k] = g.P[k] = P[ax];
+      Launch L{};
+      L.y_tx = 8;
+      if (ax == 0) {
+        KB_TRY(launch_xfwd<double2>(g, d, L, c, c, 6 * vol / P[0], B.st));
+      } else {
+        g.P[0] = ax == 1 ? P[0] : P[0] * P[1];
+        g.sc[2] = ax == 1 ? P[2] : 1;
+        KB_TRY(launch_y<double2>(g, d, L, false, c, c, 0, ax == 1 ? 6LL * P[2] : 6, 0, 0, B.st));
+      }
+      continue;
+    }
     AxisPlan* pl_d;
     if ((s = B.alloc(&pl_d, 1)) != GILA_OK) return s;
     KB_TRY(cudaMemcpyAsync(pl_d, &pl, sizeof(pl), cudaMemcpyHostToDevice, B.st));
@@ -1584,10 +1932,11 @@ static gila_status ext_circulant(Build& B, const HVol& t, const HVol& sv, const 
     fp.split[d] = (int)t.cel[d];
     fp.touch[d] = contact ? CNT_TOL + (rd(t.scl[d]) + rd(sv.scl[d])) / 2.0 : -1.0;
   }
-  fp.nitems = vol;
   fp.out = crc_d;
-  fp.errflag = err_d;
-  if ((s = run_far(B, fp, g_d)) != GILA_OK) return s;
+  Cub cub;
+  if ((s = cub_alloc(B, vol, g_d, err_d, &cub)) != GILA_OK) return s;
+  if ((s = cub_reset(B, cub)) != GILA_OK) return s;
+  if ((s = run_far(B, cub, fp, vol)) != GILA_OK) return s;
   if (contact) {
     // genCntVol (src/glaGen.jl:308-318) and its self circulant
     int64_t cel[3];
