@@ -1584,32 +1584,49 @@ struct DBuf {
     if (e__ != cudaSuccess) return ::gila::cuda_fail(e__, #expr); \
   } while (0)
 
+// Scratch of one build: parts of a few large blocks.  Every device allocation
+// above a megabyte costs 0.35 ms and its release 0.3 ms, and the build's dozen
+// buffers took longer than its kernels (32^3 self operator: 6 of 9.6 ms).
 struct Build {
   Ctx* ctx;
   cudaStream_t st;
   Z f;
   int ord;
-  Consts* q_d = nullptr;  // in `keep`
+  Consts* q_d = nullptr;  // in a block
+  size_t block_bytes = size_t(32) << 20;  // of the next block, at least
   std::vector<DBuf*> keep;
+  size_t off = 0, cap = 0;  // of the last block
   ~Build() {
     for (auto* b : keep) delete b;
   }
-  // frees the buffers allocated after `mark` (the stream is synchronised
-  // first: kernels in flight may still use them)
-  void release_from(size_t mark) {
-    if (keep.size() <= mark) return;
+  struct Mark {
+    size_t blocks, off, cap;
+  };
+  Mark mark() const { return Mark{keep.size(), off, cap}; }
+  // gives back what was allocated after the mark (the stream is synchronised
+  // first: kernels in flight may still use it)
+  void release_to(const Mark& m) {
     cudaStreamSynchronize(st);
-    while (keep.size() > mark) {
+    while (keep.size() > m.blocks) {
       delete keep.back();
       keep.pop_back();
     }
+    off = m.off;
+    cap = m.cap;
   }
   template <typename T>
   gila_status alloc(T** out, size_t n) {
-    DBuf* b = new DBuf;
-    keep.push_back(b);
-    KB_TRY(dev_malloc(&b->p, n * sizeof(T) + 16));
-    *out = static_cast<T*>(b->p);
+    const size_t bytes = (n * sizeof(T) + 16 + 255) / 256 * 256;
+    if (off + bytes > cap) {
+      DBuf* b = new DBuf;
+      keep.push_back(b);
+      off = cap = 0;
+      const size_t want = std::max(bytes, block_bytes);
+      KB_TRY(dev_malloc(&b->p, want));
+      cap = want;
+    }
+    *out = reinterpret_cast<T*>(static_cast<unsigned char*>(keep.back()->p) + off);
+    off += bytes;
     return GILA_OK;
   }
 };
@@ -1689,9 +1706,16 @@ struct Cub {
   const PairGeo* g;
   int* err;
 };
+static size_t cub_items(int64_t nitems) {
+  return (size_t)std::min<int64_t>(std::max<int64_t>(nitems, 1), kFarChunk) + 8;
+}
+static size_t cub_bytes(int64_t nitems) {
+  return cub_items(nitems) * (sizeof(Rec) + 24 * sizeof(Z) + 3 * 24 * sizeof(Unit)) +
+         (size_t)kWarps2 * kCap2 * kRegBytes + 8 * 512;
+}
 static gila_status cub_alloc(Build& B, int64_t nitems, const PairGeo* g_d, int* err_d, Cub* q) {
   gila_status s;
-  const size_t n = (size_t)std::min<int64_t>(std::max<int64_t>(nitems, 1), kFarChunk) + 8;
+  const size_t n = cub_items(nitems);
   q->g = g_d;
   q->err = err_d;
   if ((s = B.alloc(&q->L.rec, n)) != GILA_OK) return s;
@@ -2013,12 +2037,19 @@ gila_status build_kernel(Core& c) {
   if (B.ord > kMaxOrd) return fail(GILA_ERR_ARG, "intOrd above 64 is not supported");
   gila_status s;
   {
+    // one block for the circulant, the field and the work lists
+    const int64_t pv = (int64_t)c.geom.P[0] * c.geom.P[1] * c.geom.P[2], items = c.self ? pv / 8 : pv;
+    B.block_bytes = (size_t)(6 * pv * (int64_t)sizeof(Z) + (c.self ? 6 * items * (int64_t)sizeof(Z) : 0)) +
+                    cub_bytes(items) + (size_t(4) << 20);
+  }
+  {
     Consts q;
     q.ord = B.ord;
     gauss_legendre(B.ord, q.x, q.w);
     q.f = B.f;
     if ((s = B.alloc(&B.q_d, 1)) != GILA_OK) return s;
     KB_TRY(cudaMemcpyAsync(B.q_d, &q, sizeof(q), cudaMemcpyHostToDevice, B.st));
+    B.block_bytes = size_t(32) << 20;  // of any further block
   }
   KB_TRY(cudaMemcpyToSymbolAsync(c_sng_cor, SNG_COR, sizeof(SNG_COR), 0, cudaMemcpyHostToDevice, B.st));
   KB_TRY(cudaMemcpyToSymbolAsync(c_sng_mask, SNG_MASK, sizeof(SNG_MASK), 0, cudaMemcpyHostToDevice, B.st));
@@ -2036,7 +2067,7 @@ gila_status build_kernel(Core& c) {
   const size_t per = (size_t)g.tru[0] * g.tru[1] * g.tru[2] * 6 * 8;  // elements per target partition
   KB_TRY(dev_malloc(&c.ker, per * parT * cs));
   c.ker_bytes = per * parT * cs;
-  const size_t mark = B.keep.size();
+  const Build::Mark mark = B.mark();
   for (int tp = 0; tp < parT; ++tp) {
     if (c.self) {
       if ((s = self_circulant(B, t, crc_d, err_d)) != GILA_OK) return s;
@@ -2054,7 +2085,7 @@ gila_status build_kernel(Core& c) {
       k_extract<float2><<<1184, 256, 0, B.st>>>(crc_d, P[0], P[1], P[2], g.tru[0], g.tru[1], g.tru[2],
                                                static_cast<float2*>(c.ker) + per * tp, err_d + 1);
     KB_TRY(cudaGetLastError());
-    B.release_from(mark);  // this partition's cubature scratch
+    if (tp + 1 < parT) B.release_to(mark);  // this partition's cubature scratch
   }
   int flags[2];
   KB_TRY(cudaMemcpyAsync(flags, err_d, sizeof(flags), cudaMemcpyDeviceToHost, B.st));
@@ -2082,6 +2113,7 @@ gila_status weak_integrals(Ctx* ctx, const Rat scl[3], kb::Z f, int ord, double 
     B.st = st;
     B.f = f;
     B.ord = ord;
+    B.block_bytes = size_t(4) << 20;
     Consts q;
     q.ord = ord;
     gauss_legendre(ord, q.x, q.w);
