@@ -312,48 +312,93 @@ constexpr MxSched mx_search(int P, int rmax, int last_max, int stage_cost) {
   return m.best;
 }
 
-// MXK_XY: x and y passes; MXK_Z: fused z pass
+// MXK_XY: x and y passes; MXK_Z: fused z pass, whose last radix three
+// components share a thread's registers
 enum { MXK_XY = 0, MXK_Z = 1 };
-#ifndef GILA_MX_RMAX
-#define GILA_MX_RMAX 10
-#endif
-#ifndef GILA_MX_ZRMAX
-#define GILA_MX_ZRMAX 10
-#endif
 #ifndef GILA_MX_STAGE
 #define GILA_MX_STAGE 400
 #endif
+constexpr MxSched mx_sched(int P, int kind) {
+  return mx_search(P, P <= 100 ? 10 : 16, kind == MXK_Z ? 4 : 16, GILA_MX_STAGE);
+}
 template <int P, int KIND> struct MxPlan {
-  // (z passes past 256: radices up to 16, so that three components' threads
-  // leave 96 registers and more to each)
-  static constexpr MxSched s = mx_search(P, KIND == MXK_Z ? (P > 256 ? 16 : GILA_MX_ZRMAX) : GILA_MX_RMAX,
-                                         KIND == MXK_Z ? 4 : 16, GILA_MX_STAGE);
+  static constexpr MxSched s = mx_sched(P, KIND);
 };
 // radix and span of stage S, in reversed order for the z pass's inverse
-template <int P, int KIND, bool REV> constexpr int mx_r(int S) {
-  return REV ? MxPlan<P, KIND>::s.r[MxPlan<P, KIND>::s.n - 1 - S] : MxPlan<P, KIND>::s.r[S];
-}
-template <int P, int KIND, bool REV> constexpr int mx_span(int S) {
+constexpr int mx_sr(const MxSched& s, bool rev, int S) { return rev ? s.r[s.n - 1 - S] : s.r[S]; }
+constexpr int mx_sspan(const MxSched& s, bool rev, int S) {
   int ns = 1;
-  for (int k = 0; k < S; ++k) ns *= mx_r<P, KIND, REV>(k);
+  for (int k = 0; k < S; ++k) ns *= mx_sr(s, rev, k);
   return ns;
 }
+template <int P, int KIND, bool REV> constexpr int mx_r(int S) { return mx_sr(MxPlan<P, KIND>::s, REV, S); }
+template <int P, int KIND, bool REV> constexpr int mx_span(int S) { return mx_sspan(MxPlan<P, KIND>::s, REV, S); }
 
+// Twiddle tables of a length, behind the P entries w^m of its table: for each
+// stage after the first of the x / y plan, of the z plan and of the reversed z
+// plan the factors w^(q jm P / (NS R)) as [q - 1][jm], so that neighbouring
+// threads (neighbouring jm) load neighbouring entries.  From the plain table
+// they load entries q P / (NS R) apart, a cache line each: in the x passes the
+// twiddles then take more of the load pipe than the data.
+constexpr int mx_tw_stages(const MxSched& s, bool rev, int S) {  // entries of stages 1 .. S - 1
+  int n = 0;
+  for (int k = 1; k < S; ++k) n += (mx_sr(s, rev, k) - 1) * mx_sspan(s, rev, k);
+  return n;
+}
+constexpr int mx_tw_base(int P, int kind, bool rev) {
+  int b = P;
+  if (kind == MXK_Z) b += mx_tw_stages(mx_sched(P, MXK_XY), false, mx_sched(P, MXK_XY).n);
+  if (kind == MXK_Z && rev) b += mx_tw_stages(mx_sched(P, MXK_Z), false, mx_sched(P, MXK_Z).n);
+  return b;
+}
+constexpr int mx_tw_len(int P) {
+  return mx_tw_base(P, MXK_Z, true) + mx_tw_stages(mx_sched(P, MXK_Z), true, mx_sched(P, MXK_Z).n);
+}
+template <int P, int KIND, bool REV, int S> struct MxTw {
+  static constexpr int off = mx_tw_base(P, KIND, REV) + mx_tw_stages(MxPlan<P, KIND>::s, REV, S);
+};
+// exponents of the entries P .. mx_tw_len(P) - 1 (host)
+template <typename F>
+inline void mx_tw_fill(int P, const F& put) {
+  int at = P;
+  for (int t = 0; t < 3; ++t) {
+    const MxSched s = mx_sched(P, t == 0 ? MXK_XY : MXK_Z);
+    const bool rev = t == 2;
+    for (int k = 1; k < s.n; ++k) {
+      const int R = mx_sr(s, rev, k), NS = mx_sspan(s, rev, k), st = P / (NS * R);
+      for (int q = 1; q < R; ++q)
+        for (int jm = 0; jm < NS; ++jm) put(at++, (int)((long)q * jm * st % P));
+    }
+  }
+}
+
+// Shared-memory line of a plan: element i sits at i + i / R0 where the first
+// radix R0 is even, at i where it is odd, so that the first stage's stores (R0
+// apart) start on different banks; its length in elements.
+template <int P, int KIND> GILA_HD int mx_pad(int i) {
+  constexpr int r0 = MxPlan<P, KIND>::s.r[0];
+  return r0 % 2 == 0 ? i + (int)((unsigned)i / (unsigned)r0) : i;
+}
+template <int P, int KIND> constexpr int mx_line_len() {
+  constexpr int r0 = MxPlan<P, KIND>::s.r[0];
+  return r0 % 2 == 0 ? P + P / r0 : P;
+}
 // ----------------------------------------------------------------- stages
-// Twiddles w^(q step), q = 1 .. R-1.  FP64: every fourth from the table, the
-// others one product away from those (two for w^3): a table load costs as
-// much of the load/store pipe as a data access.  FP32: all from the table.
-template <int R, bool INV, typename W>
-__device__ __forceinline__ void mx_twiddles(const W* __restrict__ tw, int step, W* w) {
+// Twiddles q = 1 .. R-1 of a stage of span NS from its table (at jm).  FP64:
+// every fourth loaded, the others one product away from those (two for w^3):
+// a load costs as much of the load/store pipe as a data access.  FP32: all
+// loaded.
+template <int R, int NS, bool INV, typename W>
+__device__ __forceinline__ void mx_twiddles(const W* __restrict__ tw, W* w) {
   if constexpr (sizeof(W) == 16) {
-    if constexpr (R > 1) w[1] = twid<INV>(tw, step);
+    if constexpr (R > 1) w[1] = twid<INV>(tw, 0);
     if constexpr (R > 2) w[2] = cmul(w[1], w[1]);
     if constexpr (R > 3) w[3] = cmul(w[2], w[1]);
 #pragma unroll
-    for (int q = 4; q < R; ++q) w[q] = q % 4 == 0 ? twid<INV>(tw, q * step) : cmul(w[q - q % 4], w[q % 4]);
+    for (int q = 4; q < R; ++q) w[q] = q % 4 == 0 ? twid<INV>(tw, (q - 1) * NS) : cmul(w[q - q % 4], w[q % 4]);
   } else {
 #pragma unroll
-    for (int q = 1; q < R; ++q) w[q] = twid<INV>(tw, q * step);
+    for (int q = 1; q < R; ++q) w[q] = twid<INV>(tw, (q - 1) * NS);
   }
 }
 
@@ -384,7 +429,7 @@ __device__ __forceinline__ void mx_stage(int j0, const typename MxOf<V>::W* __re
       const int jm = NS == 1 ? 0 : (NS == TPL ? j : j % NS);
       if constexpr (NS > 1) {
         W w[R];
-        mx_twiddles<R, INV>(tw, jm * (P / (NS * R)), w);
+        mx_twiddles<R, NS, INV>(tw + MxTw<P, KIND, REV, S>::off + jm, w);
 #pragma unroll
         for (int r = 1; r < R; ++r) v[k][r] = vmul(v[k][r], w[r]);
       }

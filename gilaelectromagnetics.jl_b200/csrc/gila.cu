@@ -14,7 +14,9 @@
 #include <string>
 #include <vector>
 
+#include "fft_mx.cuh"
 #include "internal.h"
+#include "matvec_mx.cuh"
 
 namespace gila {
 
@@ -195,23 +197,30 @@ gila_status twiddle_table(Ctx* ctx, int P, gila_dtype dt, const void** out) {
     *out = it->second;
     return GILA_OK;
   }
-  // w_P^m = exp(-2 pi i m / P); angle reduced to the first octant for accuracy
-  std::vector<double> re(P), im(P);
+  // w_P^m = exp(-2 pi i m / P); angle reduced to the first octant for
+  // accuracy; behind them the stage tables of the mixed-radix passes
+  const int len = mx_ops<double2>(P) ? mx_tw_len(P) : P;
+  std::vector<double> re(len), im(len);
   for (int m = 0; m < P; ++m) {
     const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)P;
     re[m] = (double)cosl(a);
     im[m] = (double)sinl(a);
   }
+  if (len > P)
+    mx_tw_fill(P, [&](int at, int m) {
+      re[at] = re[m];
+      im[at] = im[m];
+    });
   void* d = nullptr;
-  const size_t bytes = (size_t)P * csize(dt);
+  const size_t bytes = (size_t)len * csize(dt);
   GILA_CUDA_TRY(dev_malloc(&d, bytes));
   if (dt == GILA_C128) {
-    std::vector<double2> h(P);
-    for (int m = 0; m < P; ++m) h[m] = make_double2(re[m], im[m]);
+    std::vector<double2> h(len);
+    for (int m = 0; m < len; ++m) h[m] = make_double2(re[m], im[m]);
     GILA_CUDA_TRY(cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice));
   } else {
-    std::vector<float2> h(P);
-    for (int m = 0; m < P; ++m) h[m] = make_float2((float)re[m], (float)im[m]);
+    std::vector<float2> h(len);
+    for (int m = 0; m < len; ++m) h[m] = make_float2((float)re[m], (float)im[m]);
     GILA_CUDA_TRY(cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice));
   }
   ctx->tw_cache[key] = d;

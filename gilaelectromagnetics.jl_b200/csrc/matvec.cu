@@ -88,7 +88,7 @@ static bool ct_len(int P) {
 
 std::vector<int> ct_tiles(int cs, int P, bool z) {
   std::vector<int> v;
-  if (!ct_len(P)) return v;
+  if (!ct_len(P) || (!z && P % 3 == 0)) return v;  // 96, 192, 384: z only
   for (int tx : kTileSet)
     if (z ? ct_z_ok(cs, P, tx) : ct_y_ok(cs, P, tx)) v.push_back(tx);
   return v;

@@ -2267,6 +2267,12 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<sizeof(C)>(P), P)) k_xinv
 
 // Lengths with specialised kernels.
 #define GILA_CT_SIZES(X) X(64) X(96) X(128) X(192) X(256) X(384) X(512)
+// of them, lengths with x and y kernels: at 96, 192 and 384 the mixed-radix x
+// and y passes are faster (both directions, F64: 0.340 -> 0.296 ms at 192 with
+// four vectors of 96x96x48, 0.786 -> 0.589 ms at 384 with 192x192x96; F32: 0.197
+// -> 0.165 and 0.440 -> 0.374 ms), their z passes slower (0.318 -> 0.454 ms)
+#define GILA_CT_XY_SIZES(X) X(64) X(128) X(256) X(512)
+static bool ct_has_xy(int P) { return P == 64 || P == 128 || P == 256 || P == 512; }
 static bool ct_has(int P) {
 #define GILA_CT_CASE(n) if (P == n) return true;
   GILA_CT_SIZES(GILA_CT_CASE)
@@ -2408,7 +2414,7 @@ cudaError_t launch_xfwd(const Geom& g, const DevOp<C>& d, const Launch& L, const
   p.M = L.xf_lines;
   p.rows = rows;
   p.nind = make_fdiv((uint32_t)p.nin);
-  if (ct_has(p.P)) {
+  if (ct_has_xy(p.P)) {
 #define GILA_CT_XF(n)                                                                  \
   if constexpr (sizeof(C) == 8) {                                                      \
     if (p.P == n && zpair()) {                                                         \
@@ -2459,7 +2465,7 @@ cudaError_t launch_xfwd(const Geom& g, const DevOp<C>& d, const Launch& L, const
       GILA_LAUNCH(false, (k_xfwd_ct<C, n, false>), p);                                 \
     return cudaGetLastError();                                                         \
   }
-    GILA_CT_SIZES(GILA_CT_XF)
+    GILA_CT_XY_SIZES(GILA_CT_XF)
 #undef GILA_CT_XF
   }
   if (const MxOps<C>* o = mx_ops<C>(p.P)) return o->xfwd(p, st);
@@ -2477,7 +2483,7 @@ cudaError_t launch_xfwd(const Geom& g, const DevOp<C>& d, const Launch& L, const
 template <typename C, bool INV>
 static cudaError_t launch_y_one(const YParams<C>& p, bool mx, int T, size_t sm, int64_t blocks, bool rev, bool gform,
                                 cudaStream_t st) {
-  if (ct_has(p.P)) {
+  if (ct_has_xy(p.P)) {
 #define GILA_CT_Y2(n, tx)                                  \
   if constexpr (ct_y_ok(sizeof(C), n, tx)) {               \
     if (p.P == n && p.TX == tx) {                          \
@@ -2522,7 +2528,7 @@ static cudaError_t launch_y_one(const YParams<C>& p, bool mx, int T, size_t sm, 
     }                                                      \
   }
 #define GILA_CT_Y(n) GILA_CT_Y2(n, 4) GILA_CT_Y2(n, 8) GILA_CT_Y2(n, 16)
-    GILA_CT_SIZES(GILA_CT_Y)
+    GILA_CT_XY_SIZES(GILA_CT_Y)
 #undef GILA_CT_Y
 #undef GILA_CT_Y2
     return cudaErrorInvalidConfiguration;
@@ -2592,7 +2598,7 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
   p.q0 = q0;
   p.src_sub = src_sub;
   p.dst_sub = dst_sub;
-  if (ct_has(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.y_tx, false);
+  if (ct_has_xy(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.y_tx, false);
   const MxOps<C>* const mx = mx_pairs_ok<C>(p.Px, src, dst) ? mx_ops<C>(p.P) : nullptr;
   if (mx) p.TX = mx->y_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
@@ -2604,7 +2610,7 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
     if (!chunk_y_tiles(p.Px, txz, p.TX, *ch, p.lo0, p.nlo, p.hi0, p.nt)) return cudaErrorInvalidValue;
   }
   if (mx) return mx->y(p, inv, (int64_t)p.nt * nq, st);
-  const int T = ct_has(p.P) ? ct_threads(p.TX, p.P) : pass_threads(d.plan[1], p.TX);
+  const int T = ct_has_xy(p.P) ? ct_threads(p.TX, p.P) : pass_threads(d.plan[1], p.TX);
   if (T > 512) return cudaErrorInvalidConfiguration;
   const size_t sm = (size_t)p.TX * p.P * sizeof(C);
   const bool mixed = is_mixed(d.plan[1]);
@@ -2654,7 +2660,8 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
     p.ax[k].fo = (g.tc[k] + 1) / 2;
   }
   if (ct_has(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.z_tx, true);
-  const MxOps<C>* const mx = g.parT == 1 && mx_pairs_ok<C>(p.Px, B, B) ? mx_ops<C>(p.P) : nullptr;
+  const MxOps<C>* const mx =
+      g.parT == 1 && !ct_has(p.P) && mx_pairs_ok<C>(p.Px, B, B) ? mx_ops<C>(p.P) : nullptr;
   if (mx) p.TX = mx->z_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
   p.md = make_fdiv((uint32_t)p.TX);
@@ -2736,7 +2743,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
 template <typename C, bool AXPBY>
 static cudaError_t launch_xinv_one(const XiParams<C>& p, bool mx, int T, size_t sm, int64_t blocks, bool rev,
                                    bool gform, cudaStream_t st) {
-  if (ct_has(p.P)) {
+  if (ct_has_xy(p.P)) {
 #define GILA_CT_XI(n)                                                    \
   if constexpr (sizeof(C) == 8 && !AXPBY) {                              \
     if (p.P == n && !p.part_scatter && zpair()) {                        \
@@ -2781,7 +2788,7 @@ static cudaError_t launch_xinv_one(const XiParams<C>& p, bool mx, int T, size_t 
       GILA_LAUNCH(false, (k_xinv_ct<C, n, AXPBY, false>), p);            \
     return cudaSuccess;                                                  \
   }
-    GILA_CT_SIZES(GILA_CT_XI)
+    GILA_CT_XY_SIZES(GILA_CT_XI)
 #undef GILA_CT_XI
   }
   if (mx)
@@ -2826,16 +2833,15 @@ cudaError_t launch_xinv(const Geom& g, const DevOp<C>& d, const Launch& L, const
   p.alpha = alpha;
   p.beta = beta;
   p.pd = make_fdiv((uint32_t)p.P);
-  if (ct_has(p.P)) {
+  if (ct_has_xy(p.P)) {
     int m = 1;
 #define GILA_CT_XL(n) if (p.P == n) m = ct_xlines<sizeof(C)>(n);
-    GILA_CT_SIZES(GILA_CT_XL)
+    GILA_CT_XY_SIZES(GILA_CT_XL)
 #undef GILA_CT_XL
     p.M = m;
   }
-  if (!p.part_scatter)
-    if (const MxOps<C>* o = mx_ops<C>(p.P)) return o->xinv(p, axpby, st);
-  const int T = ct_has(p.P) ? ct_threads(p.M, p.P) : pass_threads(d.plan[0], p.M);
+  if (const MxOps<C>* o = mx_ops<C>(p.P)) return o->xinv(p, axpby, st);
+  const int T = ct_has_xy(p.P) ? ct_threads(p.M, p.P) : pass_threads(d.plan[0], p.M);
   if (T > 512) return cudaErrorInvalidConfiguration;
   const size_t sm = (size_t)p.M * row_stride(p.P) * sizeof(C);
   const bool mx = is_mixed(d.plan[0]);
@@ -2907,7 +2913,7 @@ template <typename C>
 int kx_chunks(const Geom& g, const DevOp<C>& d, const Launch& L, int nrhs) {
   const int want = kx_chunks_wanted();
   if (want < 2 || !d.pst[0] || !d.pst[1] || !d.pjoin || g.parT != 1) return 0;
-  if (!ct_has(g.P[1]) || !ct_has(g.P[2])) return 0;
+  if (!ct_has_xy(g.P[1]) || !ct_has(g.P[2])) return 0;
   const Work w = work_sizes(g);
   const int64_t fwd = 3LL * g.sc[2] * nrhs, inv = 3LL * g.tc[2] * nrhs;
   if ((int64_t)w.zb != g.sc[2] || (int64_t)w.zb != g.tc[2] || w.slab_planes < fwd || w.slab_planes < inv) return 0;

@@ -2,5 +2,5 @@
 #include "matvec_mx_impl.cuh"
 
 namespace gila {
-GILA_MX_PART(3, 6, 20, 50, 84, 144, 200, 288, 360, 486)
+GILA_MX_PART(3, 192, 6, 20, 50, 84, 144, 200, 288, 360, 486)
 }  // namespace gila

@@ -2,5 +2,5 @@
 #include "matvec_mx_impl.cuh"
 
 namespace gila {
-GILA_MX_PART(5, 28, 42, 98, 126, 216, 270, 392, 450)
+GILA_MX_PART(5, 96, 28, 42, 98, 126, 216, 270, 392, 450)
 }  // namespace gila

@@ -75,19 +75,18 @@ __device__ __forceinline__ void mx_line(int j0, const typename MxOf<V>::W* __res
 
 // -------------------------------------------------------------------- x
 // A thread group of TPB threads per row (ComplexF32: per row pair), any
-// number of groups per block; a row's elements sit at i + i / 8 of its
-// shared-memory line, as in the other x passes.
+// number of groups per block; a row is one padded shared-memory line.
 template <typename C, int P>
 __global__ void __launch_bounds__(256) k_xfwd_mx(const XfParams<C> p) {
   using V = typename MxElem<C>::V;
-  constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = P + (P + 7) / 8;
+  constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = mx_line_len<P, MXK_XY>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int l = (int)threadIdx.x / TPB, j0 = (int)threadIdx.x % TPB;
   V* const sm = reinterpret_cast<V*>(smem_raw) + l * LS;
   const int nin = p.nin;
   const int64_t u = (int64_t)blockIdx.x * p.M + l;
-  auto ld = [=](int i) -> V { return mx_ldg(sm + i + (i >> 3)); };
-  auto st = [=](int i, V v) { mx_st(sm + i + (i >> 3), v); };
+  auto ld = [=](int i) -> V { return mx_ldg(sm + mx_pad<P, MXK_XY>(i)); };
+  auto st = [=](int i, V v) { mx_st(sm + mx_pad<P, MXK_XY>(i), v); };
   if constexpr (sizeof(C) == 16) {
     const bool ok = u < p.rows;
     const C* const src = p.in + u * nin;
@@ -116,10 +115,12 @@ __global__ void __launch_bounds__(256) k_xfwd_mx(const XfParams<C> p) {
   }
 }
 
-template <typename C, int P>
-__global__ void __launch_bounds__(256) k_xinv_mx(const XiParams<C> p, const int axpby) {
+// SCAT: target partitions interleaved into the full target volume (its index
+// arithmetic in the common form cost 20% of the pass)
+template <typename C, int P, bool SCAT>
+__global__ void __launch_bounds__(256) k_xinv_mx(const __grid_constant__ XiParams<C> p, const int axpby) {
   using V = typename MxElem<C>::V;
-  constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = P + (P + 7) / 8;
+  constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = mx_line_len<P, MXK_XY>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int l = (int)threadIdx.x / TPB, j0 = (int)threadIdx.x % TPB;
   V* const sm = reinterpret_cast<V*>(smem_raw) + l * LS;
@@ -130,9 +131,26 @@ __global__ void __launch_bounds__(256) k_xinv_mx(const XiParams<C> p, const int 
   const C *const ls_in = p.ls_in, *const ls_chi = p.ls_chi;
   const int64_t ls_chi_rs = p.ls_chi_rs, rows = p.rows, g_off = p.g_off;
   const FDiv rows_rhs = p.rows_rhs, rows_zy = p.rows_zy;
+  const XiParams<C>* const pp = &p;
   auto put = [=](int64_t g, int i, C v) {
     if (g >= rows || i >= nout) return;
-    const int64_t gg = g + g_off, o = gg * nout + i;
+    const int64_t gg = g + g_off;
+    int64_t o = gg * nout + i;
+    if constexpr (SCAT) {
+      // gg = ((rhs*parT + t)*3 + c)*tz + z)*ty + y (mrgPrtDev!)
+      int64_t q = gg;
+      const int y = (int)(q % pp->ty);
+      q /= pp->ty;
+      const int z = (int)(q % pp->tz);
+      q /= pp->tz;
+      const int c = (int)(q % 3);
+      q /= 3;
+      const int t = (int)(q % pp->parT);
+      const int64_t rhs = q / pp->parT;
+      const int64_t X = (int64_t)i * pp->tdiv[0] + pp->toff[t][0], Y = (int64_t)y * pp->tdiv[1] + pp->toff[t][1],
+                    Zz = (int64_t)z * pp->tdiv[2] + pp->toff[t][2];
+      o = (((rhs * 3 + c) * pp->full[2] + Zz) * pp->full[1] + Y) * pp->full[0] + X;
+    }
     if (axpby)
       out[o] = cadd(cmul(alpha, v), cmul(beta, out[o]));
     else if (ls)
@@ -140,8 +158,8 @@ __global__ void __launch_bounds__(256) k_xinv_mx(const XiParams<C> p, const int 
     else
       out[o] = v;
   };
-  auto ld = [=](int i) -> V { return mx_ldg(sm + i + (i >> 3)); };
-  auto st = [=](int i, V v) { mx_st(sm + i + (i >> 3), v); };
+  auto ld = [=](int i) -> V { return mx_ldg(sm + mx_pad<P, MXK_XY>(i)); };
+  auto st = [=](int i, V v) { mx_st(sm + mx_pad<P, MXK_XY>(i), v); };
   if constexpr (sizeof(C) == 16) {
     const bool ok = u < rows;
     const C* const src = p.A + u * P;
@@ -210,7 +228,14 @@ __global__ void __launch_bounds__(mx_y_threads<P>(), mx_blocks(mx_y_threads<P>()
 // -------------------------------------------------------------------- z
 // kx elements per tile: 128-byte rows while three components' lines leave
 // room for two blocks or more per SM, else half of that
-template <int P> constexpr int mx_z_tx() { return P <= 192 ? 8 : 4; }
+#ifndef GILA_MX_ZTX8
+#define GILA_MX_ZTX8 192
+#endif
+template <int P> constexpr int mx_z_tx() { return P <= GILA_MX_ZTX8 ? 8 : 4; }
+// z lines of a tile in shared memory: rows of TX elements, at tiles of 4 padded
+// like an x line (two rows share a quarter-warp's banks)
+template <int P> GILA_HD int mx_z_row(int i) { return mx_z_tx<P>() == 8 ? i : mx_pad<P, MXK_Z>(i); }
+template <int P> constexpr int mx_z_rows() { return mx_z_tx<P>() == 8 ? P : mx_line_len<P, MXK_Z>(); }
 template <int P> constexpr int mx_z_threads() { return 3 * mx_z_tx<P>() * MxPlan<P, MXK_Z>::s.tpb; }
 
 // the 3x3 products of one frequency of an element's column(s)
@@ -240,7 +265,8 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = (int)threadIdx.x % TX, q = (int)threadIdx.x / TX, c = q / TPB, j0 = q % TPB;
   V* const smt = reinterpret_cast<V*>(smem_raw) + t;  // [c][z][t]
-  V* const smc = smt + c * (P * TX);
+  constexpr int ZR = mx_z_rows<P>();
+  V* const smc = smt + c * (ZR * TX);
   const int nrhs = p.nrhs, Px = p.Px, Py = p.Py, nin = p.nin, nout = p.nout;
   const int rhs = blockIdx.x % nrhs;
   const int rest = blockIdx.x / nrhs;
@@ -252,8 +278,8 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
   const int64_t plane = (int64_t)Py * Px;
   C* const Bb = p.B + (int64_t)rhs * 3 * p.zb * plane + (int64_t)ky * Px + kx;
   const W* const tw = p.tw;
-  auto ld = [=](int i) -> V { return mx_ldg(smc + i * TX); };
-  auto st = [=](int i, V v) { mx_st(smc + i * TX, v); };
+  auto ld = [=](int i) -> V { return mx_ldg(smc + mx_z_row<P>(i) * TX); };
+  auto st = [=](int i, V v) { mx_st(smc + mx_z_row<P>(i) * TX, v); };
   auto sync = [] { __syncthreads(); };
   auto none = [] {};
   {
@@ -332,10 +358,10 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
-      for (int r = 0; r < RL; ++r) v[d][r] = mx_ldg(smt + (d * P + j + r * TPL) * TX);
+      for (int r = 0; r < RL; ++r) v[d][r] = mx_ldg(smt + (d * ZR + mx_z_row<P>(j + r * TPL)) * TX);
     {
       W w[RL];
-      mx_twiddles<RL, false>(tw, j, w);
+      if constexpr (N > 1) mx_twiddles<RL, TPL, false>(tw + MxTw<P, MXK_Z, false, N - 1>::off + j, w);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         if constexpr (N > 1) {
@@ -361,14 +387,14 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
     for (int d = 0; d < 3; ++d) {
       Dft<RL, true>::run(v[d]);
 #pragma unroll
-      for (int r = 0; r < RL; ++r) mx_st(smt + (d * P + j + r * TPL) * TX, v[d][r]);
+      for (int r = 0; r < RL; ++r) mx_st(smt + (d * ZR + mx_z_row<P>(j + r * TPL)) * TX, v[d][r]);
     }
   }
   __syncthreads();
   // inverse stages in reversed order; the first reads through the fused
   // stage's permutation (input i in slot i / RL + (i % RL) P / RL)
   C* const dst = Bb + (int64_t)c * nout * plane;
-  auto ldp = [=](int i) -> V { return mx_ldg(smc + ((i / RL) + (i % RL) * TPL) * TX); };
+  auto ldp = [=](int i) -> V { return mx_ldg(smc + mx_z_row<P>((i / RL) + (i % RL) * TPL) * TX); };
   auto gst = [=](int i, V v) {
     if (ok && i < nout) mx_st(reinterpret_cast<V*>(dst + (int64_t)i * plane), v);
   };
@@ -409,7 +435,7 @@ static inline int mx_x_rows(int tpb, int64_t units) {
 
 template <typename C, int P>
 struct MxLaunch {
-  static constexpr int CW = 16 / (int)sizeof(C), LS = P + (P + 7) / 8;
+  static constexpr int CW = 16 / (int)sizeof(C), LS = mx_line_len<P, MXK_XY>();
   static constexpr int XTPB = MxPlan<P, MXK_XY>::s.tpb;
 
   static cudaError_t xfwd(const XfParams<C>& p0, cudaStream_t st) {
@@ -427,9 +453,13 @@ struct MxLaunch {
     const int64_t units = (p.rows + CW - 1) / CW;
     p.M = mx_x_rows(XTPB, units);
     const size_t sm = (size_t)p.M * LS * 16;
-    cudaError_t e = mx_smem((const void*)k_xinv_mx<C, P>, sm);
+    const unsigned blocks = (unsigned)((units + p.M - 1) / p.M);
+    cudaError_t e = mx_smem(p.part_scatter ? (const void*)k_xinv_mx<C, P, true> : (const void*)k_xinv_mx<C, P, false>, sm);
     if (e != cudaSuccess) return e;
-    k_xinv_mx<C, P><<<(unsigned)((units + p.M - 1) / p.M), p.M * XTPB, sm, st>>>(p, axpby ? 1 : 0);
+    if (p.part_scatter)
+      k_xinv_mx<C, P, true><<<blocks, p.M * XTPB, sm, st>>>(p, axpby ? 1 : 0);
+    else
+      k_xinv_mx<C, P, false><<<blocks, p.M * XTPB, sm, st>>>(p, axpby ? 1 : 0);
     return cudaGetLastError();
   }
   template <bool INV>
@@ -446,13 +476,19 @@ struct MxLaunch {
     return inv ? y_one<true>(p, units, st) : y_one<false>(p, units, st);
   }
   static cudaError_t z(const ZParams<C>& p, int64_t blocks, cudaStream_t st) {
-    const size_t sm = (size_t)3 * P * mx_z_tx<P>() * 16;
+    const size_t sm = (size_t)3 * mx_z_rows<P>() * mx_z_tx<P>() * 16;
     cudaError_t e = mx_smem((const void*)k_z_mx<C, P>, sm);
     if (e != cudaSuccess) return e;
     k_z_mx<C, P><<<(unsigned)blocks, mx_z_threads<P>(), sm, st>>>(p);
     return cudaGetLastError();
   }
-  static constexpr MxOps<C> ops{P, kMxTX * CW, mx_z_tx<P>() * CW, &xfwd, &xinv, &y, &z};
+  static constexpr auto z_or_null() -> decltype(&z) {
+    if constexpr (P == 96 || P == 192 || P == 384)
+      return nullptr;
+    else
+      return &z;
+  }
+  static constexpr MxOps<C> ops{P, kMxTX * CW, mx_z_tx<P>() * CW, &xfwd, &xinv, &y, z_or_null()};
 };
 
 template <typename C, int... P>
