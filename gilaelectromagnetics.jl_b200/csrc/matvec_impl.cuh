@@ -18,6 +18,7 @@ template <bool MX> struct StageE { static constexpr int v = MX ? kEm : kE; };
 template <typename C, bool MX>
 __global__ void __launch_bounds__(512) k_xfwd(const XfParams<C> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const AxisPlan* const pl = p.pl;
   const int P = p.P, M = p.M, nin = p.nin;
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(512) k_xfwd(const XfParams<C> p) {
 template <typename C, bool INV, bool MX>
 __global__ void __launch_bounds__(512) k_y(const YParams<C> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const AxisPlan* const pl = p.pl;
   const int Px = p.Px, TX = p.TX, nin = p.nin, nout = p.nout;
@@ -91,6 +93,7 @@ template <typename C, bool MX>
 __global__ void __launch_bounds__(512) k_z(const ZParams<C> p) {
   using T = typename Real<C>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const AxisPlan* const pl = p.pl;
   const int P = p.P;
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(512) k_z(const ZParams<C> p) {
 template <typename C, bool AXPBY, bool MX>
 __global__ void __launch_bounds__(512) k_xinv(const XiParams<C> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const AxisPlan* const pl = p.pl;
   const int P = p.P, M = p.M, nout = p.nout;
@@ -267,6 +271,7 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<sizeof(C)>(P), P)) k_xfwd
   constexpr int T = ct_threads(M, P);
   constexpr int LS = P + (P + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nin = p.nin;
   const int64_t rows = p.rows;
@@ -307,6 +312,7 @@ __global__ void __launch_bounds__(ct_threads2(ct_xlines2<8>(P), P)) k_xfwd2_ct(c
   constexpr int T = ct_threads2(M, P);
   constexpr int LS = P + (P + 7) / 8;  // float4 slots per pair row
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int nin = p.nin;
   const int64_t rows = p.rows;
@@ -347,6 +353,7 @@ __global__ void __launch_bounds__(ct_threads2(ct_xlines2<8>(P), P)) k_xinv2_ct(c
   constexpr int T = ct_threads2(M, P);
   constexpr int LS = P + (P + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int nout = p.nout;
   const int64_t rows = p.rows;
@@ -391,6 +398,7 @@ template <typename C, int P, bool INV, int TX, bool REV>
 __global__ void __launch_bounds__(ct_threads(TX, P), pow2_min_blocks(ct_threads(TX, P), P)) k_y_ct(const YParams<C> p) {
   constexpr int T = ct_threads(TX, P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int Px = p.Px, nin = p.nin, nout = p.nout;
   const int tl = blockIdx.x % p.nt;  // tile of the kx set: low range, then high range
@@ -428,6 +436,7 @@ __global__ void __launch_bounds__(ct_threads2(TX, P), pow2_min_blocks(ct_threads
   constexpr int T = ct_threads2(TX, P);
   constexpr int M2 = TX / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int Px = p.Px, nin = p.nin, nout = p.nout;
   const int tl = blockIdx.x % p.nt;  // tile of the kx set: low range, then high range
@@ -464,6 +473,7 @@ __global__ void __launch_bounds__(ct_threads(TX, P)) k_z_ct(const ZParams<C> p) 
   constexpr int T = ct_threads(TX, P);
   constexpr int CH = P * TX;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -626,6 +636,7 @@ __global__ void __launch_bounds__(ct_threads(TX, P), zf_min_blocks(ct_threads(TX
   constexpr int NTASK = TX * TPL;
   constexpr int K = (NTASK + T - 1) / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -829,6 +840,7 @@ __global__ void __launch_bounds__(zr_threads(TX, P), zr_min_blocks(zr_threads(TX
   constexpr int NA = 3 * TX * R2;  // tasks of stages A and B': (component, line, j < R2)
   constexpr int KA = (NA + T - 1) / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -1102,6 +1114,7 @@ __global__ void __launch_bounds__(ct_threads(TX, P), zf_min_blocks(ct_threads(TX
   constexpr int TPL = P / RL;
   constexpr int TPL0 = P / 8, NT0 = TX * TPL0, K0 = (NT0 + T - 1) / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -1452,6 +1465,7 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<16>(P), P)) k_xfwd_g(cons
   constexpr int T = ct_threads(M, P);
   constexpr int LS = P + (P + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nin = p.nin;
   const int64_t rows = p.rows;
@@ -1478,6 +1492,7 @@ __global__ void __launch_bounds__(ct_threads(TX, P), pow2_min_blocks(ct_threads(
   constexpr int T = ct_threads(TX, P);
   constexpr int NST = ct_nst(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int Px = p.Px, nin = p.nin, nout = p.nout;
   const int tl = blockIdx.x % p.nt;  // tile of the kx set: low range, then high range
@@ -1524,6 +1539,7 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<16>(P), P)) k_xinv_g(cons
   constexpr int LS = P + (P + 7) / 8;
   constexpr int NST = ct_nst(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nout = p.nout;
   const int64_t rows = p.rows;
@@ -1655,6 +1671,7 @@ __global__ void __launch_bounds__(ct_threads2(ct_xlines2<8>(P), P)) k_xfwd2_g(co
   constexpr int T = ct_threads2(M, P);
   constexpr int LS = P + (P + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int nin = p.nin;
   const int64_t rows = p.rows;
@@ -1688,6 +1705,7 @@ __global__ void __launch_bounds__(ct_threads2(ct_xlines2<8>(P), P)) k_xinv2_g(co
   constexpr int LS = P + (P + 7) / 8;
   constexpr int NST = ct_nst(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int nout = p.nout;
   const int64_t rows = p.rows;
@@ -1732,6 +1750,7 @@ __global__ void __launch_bounds__(ct_threads2(TX, P), pow2_min_blocks(ct_threads
   constexpr int M2 = TX / 2;
   constexpr int NST = ct_nst(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   float4* const sm = reinterpret_cast<float4*>(smem_raw);
   const int Px = p.Px, nin = p.nin, nout = p.nout;
   const int tl = blockIdx.x % p.nt;  // tile of the kx set: low range, then high range
@@ -1796,6 +1815,7 @@ __global__ void __launch_bounds__(ct_threads2(TX, P), GILA_ZF2_CAP ? zf2_min_blo
   constexpr int NTASK = M2 * TPL;
   constexpr int K = (NTASK + T - 1) / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -1995,6 +2015,7 @@ __global__ void __launch_bounds__(ct_threads2(TX, P), zf2_min_blocks(ct_threads2
   constexpr int TPL = P / RL;
   constexpr int TPL0 = P / 8, NT0 = M2 * TPL0, K0 = (NT0 + T - 1) / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nrhs = p.nrhs, ntiles = p.ntiles, Px = p.Px, Py = p.Py;
   const int nin = p.nin, nout = p.nout;
@@ -2207,6 +2228,7 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<sizeof(C)>(P), P)) k_xinv
   constexpr int T = ct_threads(M, P);
   constexpr int LS = P + (P + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   C* const sm = reinterpret_cast<C*>(smem_raw);
   const int nout = p.nout;
   const int64_t rows = p.rows;
@@ -2365,7 +2387,8 @@ static bool is_mixed(const AxisPlan& pl) {
     const void* fn__ = (const void*)KERNEL;                                                  \
     cudaError_t e__ = set_smem(fn__, sm);                                                    \
     if (e__ != cudaSuccess) return e__;                                                      \
-    KERNEL<<<(unsigned)blocks, T, sm, st>>>(__VA_ARGS__);                                    \
+    e__ = launch_pass(KERNEL, (unsigned)blocks, T, sm, st, __VA_ARGS__);                     \
+    if (e__ != cudaSuccess) return e__;                                                      \
   } while (0)
 
 // launch of an FP32 line-pair kernel with T threads (returns from the caller)
@@ -2373,8 +2396,7 @@ static bool is_mixed(const AxisPlan& pl) {
   do {                                                          \
     cudaError_t e__ = set_smem((const void*)KERNEL, SMB);       \
     if (e__ != cudaSuccess) return e__;                         \
-    KERNEL<<<(unsigned)(NB), TT, SMB, st>>>(ARG);                \
-    return cudaGetLastError();                                  \
+    return launch_pass(KERNEL, (unsigned)(NB), TT, SMB, st, ARG); \
   } while (0)
 #define GILA_LAUNCH2(KERNEL, TT, ARG) GILA_LAUNCH2_SB(KERNEL, TT, sm, blocks, ARG)
 
@@ -2383,22 +2405,19 @@ template <int P, bool REV>
 static cudaError_t run_xfwd2(const XfParams<float2>& p, int T, size_t sm, int64_t blocks, cudaStream_t st) {
   cudaError_t e = set_smem((const void*)k_xfwd2_ct<P, REV>, sm);
   if (e != cudaSuccess) return e;
-  k_xfwd2_ct<P, REV><<<(unsigned)blocks, T, sm, st>>>(p);
-  return cudaGetLastError();
+  return launch_pass(k_xfwd2_ct<P, REV>, (unsigned)blocks, T, sm, st, p);
 }
 template <int P, bool REV>
 static cudaError_t run_xinv2(const XiParams<float2>& p, int T, size_t sm, int64_t blocks, cudaStream_t st) {
   cudaError_t e = set_smem((const void*)k_xinv2_ct<P, REV>, sm);
   if (e != cudaSuccess) return e;
-  k_xinv2_ct<P, REV><<<(unsigned)blocks, T, sm, st>>>(p);
-  return cudaGetLastError();
+  return launch_pass(k_xinv2_ct<P, REV>, (unsigned)blocks, T, sm, st, p);
 }
 template <int P, bool INV, int TX, bool REV>
 static cudaError_t run_y2(const YParams<float2>& p, int T, size_t sm, int64_t blocks, cudaStream_t st) {
   cudaError_t e = set_smem((const void*)k_y2_ct<P, INV, TX, REV>, sm);
   if (e != cudaSuccess) return e;
-  k_y2_ct<P, INV, TX, REV><<<(unsigned)blocks, T, sm, st>>>(p);
-  return cudaGetLastError();
+  return launch_pass(k_y2_ct<P, INV, TX, REV>, (unsigned)blocks, T, sm, st, p);
 }
 
 template <typename C>
@@ -2599,7 +2618,7 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
   p.src_sub = src_sub;
   p.dst_sub = dst_sub;
   if (ct_has_xy(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.y_tx, false);
-  const MxOps<C>* const mx = mx_pairs_ok<C>(p.Px, src, dst) ? mx_ops<C>(p.P) : nullptr;
+  const MxOps<C>* const mx = !ct_has_xy(p.P) && mx_pairs_ok<C>(p.Px, src, dst) ? mx_ops<C>(p.P) : nullptr;
   if (mx) p.TX = mx->y_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
   p.md = make_fdiv((uint32_t)p.TX);
@@ -2687,8 +2706,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
           const void* fnr = (const void*)k_zr_ct<C, n, tx>; \
           cudaError_t er = set_smem(fnr, sm);         \
           if (er != cudaSuccess) return er;           \
-          k_zr_ct<C, n, tx><<<(unsigned)blocks, zr_threads(tx, n), sm, st>>>(p); \
-          return cudaGetLastError();                  \
+          return launch_pass(k_zr_ct<C, n, tx>, (unsigned)blocks, zr_threads(tx, n), sm, st, p); \
         }                                             \
       }                                               \
       if constexpr (sizeof(C) == 16 && zg_ok<n>()) {  \
@@ -2705,8 +2723,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
               const void* fn2 = (const void*)k_zg2_ct<n, tx>; \
               cudaError_t e2 = set_smem(fn2, sm);     \
               if (e2 != cudaSuccess) return e2;       \
-              k_zg2_ct<n, tx><<<(unsigned)blocks, T2, sm, st>>>(zp32(p)); \
-              return cudaGetLastError();              \
+              return launch_pass(k_zg2_ct<n, tx>, (unsigned)blocks, T2, sm, st, zp32(p)); \
             }                                         \
           }                                           \
           if constexpr (sizeof(C) == 8) {             \
@@ -2715,8 +2732,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
               const void* fn2 = (const void*)k_zf2_ct<n, tx>; \
               cudaError_t e2 = set_smem(fn2, sm);     \
               if (e2 != cudaSuccess) return e2;       \
-              k_zf2_ct<n, tx><<<(unsigned)blocks, T2, sm, st>>>(zp32(p)); \
-              return cudaGetLastError();              \
+              return launch_pass(k_zf2_ct<n, tx>, (unsigned)blocks, T2, sm, st, zp32(p)); \
             }                                         \
           }                                           \
           GILA_LAUNCH(false, (k_zf_ct<C, n, tx>), p); \
@@ -2840,7 +2856,8 @@ cudaError_t launch_xinv(const Geom& g, const DevOp<C>& d, const Launch& L, const
 #undef GILA_CT_XL
     p.M = m;
   }
-  if (const MxOps<C>* o = mx_ops<C>(p.P)) return o->xinv(p, axpby, st);
+  if (!ct_has_xy(p.P))
+    if (const MxOps<C>* o = mx_ops<C>(p.P)) return o->xinv(p, axpby, st);
   const int T = ct_has_xy(p.P) ? ct_threads(p.M, p.P) : pass_threads(d.plan[0], p.M);
   if (T > 512) return cudaErrorInvalidConfiguration;
   const size_t sm = (size_t)p.M * row_stride(p.P) * sizeof(C);

@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(256) k_xfwd_mx(const XfParams<C> p) {
   using V = typename MxElem<C>::V;
   constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = mx_line_len<P, MXK_XY>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   const int l = (int)threadIdx.x / TPB, j0 = (int)threadIdx.x % TPB;
   V* const sm = reinterpret_cast<V*>(smem_raw) + l * LS;
   const int nin = p.nin;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(256) k_xinv_mx(const __grid_constant__ XiParam
   using V = typename MxElem<C>::V;
   constexpr int TPB = MxPlan<P, MXK_XY>::s.tpb, LS = mx_line_len<P, MXK_XY>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   const int l = (int)threadIdx.x / TPB, j0 = (int)threadIdx.x % TPB;
   V* const sm = reinterpret_cast<V*>(smem_raw) + l * LS;
   const int nout = p.nout, ls = p.ls;
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(mx_y_threads<P>(), mx_blocks(mx_y_threads<P>()
   using V = typename MxElem<C>::V;
   constexpr int TX = kMxTX, CW = 16 / sizeof(C), TPB = MxPlan<P, MXK_XY>::s.tpb, NU = mx_y_units<P>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   const int t = (int)threadIdx.x % TX, q = (int)threadIdx.x / TX, j0 = q % TPB, un = q / TPB;
   V* const sm = reinterpret_cast<V*>(smem_raw) + un * (P * TX) + t;
   const int Px = p.Px, nin = p.nin, nout = p.nout;
@@ -263,6 +266,7 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
   constexpr int TX = mx_z_tx<P>(), CW = 16 / sizeof(C), TPB = Plan::s.tpb, N = Plan::s.n;
   constexpr int RL = mx_r<P, MXK_Z, false>(N - 1), TPL = P / RL, NJ = 3 * TPB, KF = (TPL + NJ - 1) / NJ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pass_begin();
   const int t = (int)threadIdx.x % TX, q = (int)threadIdx.x / TX, c = q / TPB, j0 = q % TPB;
   V* const smt = reinterpret_cast<V*>(smem_raw) + t;  // [c][z][t]
   constexpr int ZR = mx_z_rows<P>();
@@ -445,8 +449,7 @@ struct MxLaunch {
     const size_t sm = (size_t)p.M * LS * 16;
     cudaError_t e = mx_smem((const void*)k_xfwd_mx<C, P>, sm);
     if (e != cudaSuccess) return e;
-    k_xfwd_mx<C, P><<<(unsigned)((units + p.M - 1) / p.M), p.M * XTPB, sm, st>>>(p);
-    return cudaGetLastError();
+    return launch_pass(k_xfwd_mx<C, P>, (unsigned)((units + p.M - 1) / p.M), p.M * XTPB, sm, st, p);
   }
   static cudaError_t xinv(const XiParams<C>& p0, bool axpby, cudaStream_t st) {
     XiParams<C> p = p0;
@@ -456,11 +459,8 @@ struct MxLaunch {
     const unsigned blocks = (unsigned)((units + p.M - 1) / p.M);
     cudaError_t e = mx_smem(p.part_scatter ? (const void*)k_xinv_mx<C, P, true> : (const void*)k_xinv_mx<C, P, false>, sm);
     if (e != cudaSuccess) return e;
-    if (p.part_scatter)
-      k_xinv_mx<C, P, true><<<blocks, p.M * XTPB, sm, st>>>(p, axpby ? 1 : 0);
-    else
-      k_xinv_mx<C, P, false><<<blocks, p.M * XTPB, sm, st>>>(p, axpby ? 1 : 0);
-    return cudaGetLastError();
+    return p.part_scatter ? launch_pass(k_xinv_mx<C, P, true>, blocks, p.M * XTPB, sm, st, p, axpby ? 1 : 0)
+                          : launch_pass(k_xinv_mx<C, P, false>, blocks, p.M * XTPB, sm, st, p, axpby ? 1 : 0);
   }
   template <bool INV>
   static cudaError_t y_one(const YParams<C>& p, int64_t units, cudaStream_t st) {
@@ -469,8 +469,8 @@ struct MxLaunch {
     const size_t sm = (size_t)NU * P * kMxTX * 16;
     cudaError_t e = mx_smem((const void*)k_y_mx<C, P, INV>, sm);
     if (e != cudaSuccess) return e;
-    k_y_mx<C, P, INV><<<(unsigned)((units + NU - 1) / NU), mx_y_threads<P>(), sm, st>>>(p, (uint32_t)units);
-    return cudaGetLastError();
+    return launch_pass(k_y_mx<C, P, INV>, (unsigned)((units + NU - 1) / NU), mx_y_threads<P>(), sm, st, p,
+                       (uint32_t)units);
   }
   static cudaError_t y(const YParams<C>& p, bool inv, int64_t units, cudaStream_t st) {
     return inv ? y_one<true>(p, units, st) : y_one<false>(p, units, st);
@@ -479,8 +479,7 @@ struct MxLaunch {
     const size_t sm = (size_t)3 * mx_z_rows<P>() * mx_z_tx<P>() * 16;
     cudaError_t e = mx_smem((const void*)k_z_mx<C, P>, sm);
     if (e != cudaSuccess) return e;
-    k_z_mx<C, P><<<(unsigned)blocks, mx_z_threads<P>(), sm, st>>>(p);
-    return cudaGetLastError();
+    return launch_pass(k_z_mx<C, P>, (unsigned)blocks, mx_z_threads<P>(), sm, st, p);
   }
   static constexpr auto z_or_null() -> decltype(&z) {
     if constexpr (P == 96 || P == 192 || P == 384)
