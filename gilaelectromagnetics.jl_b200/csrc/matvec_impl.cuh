@@ -2586,6 +2586,21 @@ static bool mx_pairs_ok(int Px, const void* a, const void* b) {
   return sizeof(C) == 16 || (Px % 2 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 == 0);
 }
 
+// The length's mixed-radix z pass, or nullptr where the tuned kernels run.
+// ComplexF32 at 64: 45 us in the tuned line-pair kernel, whose last radix 8
+// fills the registers, 38 us with the mixed-radix one's 8 4 2 (two vectors of
+// 64x64x32).
+template <typename C>
+static const MxOps<C>* mx_z(int P) {
+  return !ct_has(P) || (sizeof(C) == 8 && P == 64) ? mx_ops<C>(P) : nullptr;
+}
+// kx columns per tile of a specialised z pass
+template <typename C>
+static int z_tile(int P, int want) {
+  const MxOps<C>* const o = mx_z<C>(P);
+  return o ? o->z_tx : ct_tile_pick(sizeof(C), P, want, true);
+}
+
 template <typename C>
 cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv, const C* src, C* dst, int64_t q0,
                      int64_t nq, int64_t src_sub, int64_t dst_sub, cudaStream_t st, const KxChunk* ch) {
@@ -2625,7 +2640,7 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
   p.nt = p.nlo = p.ntiles;
   p.lo0 = p.hi0 = 0;
   if (ch && ch->nts >= 0) {
-    const int txz = ct_has(g.P[2]) ? ct_tile_pick(sizeof(C), g.P[2], L.z_tx, true) : L.z_tx;
+    const int txz = ct_has(g.P[2]) ? z_tile<C>(g.P[2], L.z_tx) : L.z_tx;
     if (!chunk_y_tiles(p.Px, txz, p.TX, *ch, p.lo0, p.nlo, p.hi0, p.nt)) return cudaErrorInvalidValue;
   }
   if (mx) return mx->y(p, inv, (int64_t)p.nt * nq, st);
@@ -2679,8 +2694,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
     p.ax[k].fo = (g.tc[k] + 1) / 2;
   }
   if (ct_has(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.z_tx, true);
-  const MxOps<C>* const mx =
-      g.parT == 1 && !ct_has(p.P) && mx_pairs_ok<C>(p.Px, B, B) ? mx_ops<C>(p.P) : nullptr;
+  const MxOps<C>* const mx = g.parT == 1 && mx_pairs_ok<C>(p.Px, B, B) ? mx_z<C>(p.P) : nullptr;
   if (mx) p.TX = mx->z_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
   p.md = make_fdiv((uint32_t)p.TX);
@@ -2934,7 +2948,7 @@ int kx_chunks(const Geom& g, const DevOp<C>& d, const Launch& L, int nrhs) {
   const Work w = work_sizes(g);
   const int64_t fwd = 3LL * g.sc[2] * nrhs, inv = 3LL * g.tc[2] * nrhs;
   if ((int64_t)w.zb != g.sc[2] || (int64_t)w.zb != g.tc[2] || w.slab_planes < fwd || w.slab_planes < inv) return 0;
-  const int txz = ct_tile_pick(sizeof(C), g.P[2], L.z_tx, true);
+  const int txz = z_tile<C>(g.P[2], L.z_tx);
   const int txy = ct_tile_pick(sizeof(C), g.P[1], L.y_tx, false);
   const int Px = g.P[0];
   if (Px % txz || Px % txy || (Px / txz) % 2) return 0;
@@ -2956,7 +2970,7 @@ static cudaError_t launch_matvec_pipe(const Geom& g, const DevOp<C>& d, const La
                                       const LsEpi<C>* ls, int nch) {
   cudaError_t e;
   const int64_t fwd_planes = 3LL * g.sc[2] * nrhs, inv_planes = 3LL * g.tc[2] * nrhs;
-  const int txz = ct_tile_pick(sizeof(C), g.P[2], L.z_tx, true);
+  const int txz = z_tile<C>(g.P[2], L.z_tx);
   const int pairs = g.P[0] / txz / 2;
   if ((e = launch_xfwd<C>(g, d, L, in, A, fwd_planes * g.sc[1], st)) != cudaSuccess) return e;
   for (int c = 0; c < nch; ++c) {

@@ -42,9 +42,14 @@ constexpr int mx_blocks(int T, int regs) {
 #ifndef GILA_MX_REGS
 #define GILA_MX_REGS 96
 #endif
-#ifndef GILA_MX_ZREGS
-#define GILA_MX_ZREGS 104
-#endif
+// z pass: up to 84 registers at the short lengths, whose radices stop at 10
+// (50x40x30: 22.2 -> 20.5 us F64, 18.3 -> 16.0 us F32), 104 above (72 and 84
+// spill there: 180x140x90 F32 326 -> 441 us)
+constexpr int mx_z_regs(int P) { return P <= 100 ? 84 : 104; }
+// the next frequency's kernel values in flight while one is multiplied: F64
+// above 100 (180x140x90: 613 -> 598 us); elsewhere the registers count for more
+// (F32 180x140x90 345 -> 326 us without)
+constexpr bool mx_z_ahead(int cs, int P) { return cs == 16 && P > 100; }
 
 // stages [S, NST - 1) in place in shared memory
 template <typename V, int P, int KIND, int S, int TPB, bool INV, class Ld, class St>
@@ -257,7 +262,7 @@ struct MxCol {
 };
 
 template <typename C, int P>
-__global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>(), GILA_MX_ZREGS))
+__global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>(), mx_z_regs(P)))
     k_z_mx(const ZParams<C> p) {
   using V = typename MxElem<C>::V;
   using W = C;
@@ -357,7 +362,9 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
   for (int k = 0; k < KF; ++k) {
     const int j = q + k * NJ;
     if (j >= TPL || !ok) break;
-    MxKer<C> g = kload(j);
+    constexpr bool AHEAD = mx_z_ahead(sizeof(C), P);
+    MxKer<C> g;
+    if constexpr (AHEAD) g = kload(j);
     V v[3][RL];
 #pragma unroll
     for (int d = 0; d < 3; ++d)
@@ -378,14 +385,20 @@ __global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>()
 #pragma unroll
     for (int r = 0; r < RL; ++r) {
       MxKer<C> gn;
-      if (r + 1 < RL) gn = kload(j + (r + 1) * TPL);
+      if constexpr (AHEAD) {
+        if (r + 1 < RL) gn = kload(j + (r + 1) * TPL);
+      } else {
+        g = kload(j + r * TPL);
+      }
       if constexpr (CW == 1) {
         zmul3f(v[0][r], v[1][r], v[2][r], g.g, col.rx, ry, g.rz, s);
       } else {
         zmul3f(v[0][r].a, v[1][r].a, v[2][r].a, g.a, col.rx, ry, g.rz, s);
         zmul3f(v[0][r].b, v[1][r].b, v[2][r].b, g.b, col.rxb, ry, g.rz, s);
       }
-      if (r + 1 < RL) g = gn;
+      if constexpr (AHEAD) {
+        if (r + 1 < RL) g = gn;
+      }
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
