@@ -3,8 +3,9 @@
 // Same algorithm as fft_run in fft.cuh, but the transform length, the radix
 // schedule, the span of every stage and the line count are template
 // constants, so all index arithmetic folds to shifts / immediates and every
-// stage is unrolled.  Used for the circulant lengths the workloads use; other
-// lengths run the runtime-sized path.
+// stage is unrolled.  Used for the circulant lengths the workloads use (x and
+// y passes 64, 128, 256, 512; z passes 96, 192 and 384 too); other lengths run
+// the mixed-radix passes (fft_mx.cuh).
 #pragma once
 #include "fft.cuh"
 

@@ -6,15 +6,15 @@
 // 256x256x128, hence its JLD2 cache).  Everything stays in FP64:
 //
 //   1. weak (singular) face-pair integrals wekS / wekE / wekV: the DIRECTFN
-//      nested Gauss-Legendre sums (src/glaIntSup.jl) as block reductions,
-//      partials reduced in a fixed order (deterministic);
+//      nested Gauss-Legendre sums (src/glaIntSup.jl), one launch per kind of
+//      integral, partials reduced in a fixed order (deterministic);
 //   2. the 8 near offsets (egoFunSng!, src/glaGen.jl:350-528): corrected
 //      pairs from the weak values, the rest by cubature;
 //   3. far offsets (egoFunInn! / egoFunOut!, src/glaGen.jl:233-248,322-335):
-//      one warp per offset runs the adaptive Genz-Malik degree-7/5 cubature
-//      (the algorithm of Cubature.jl's hcubature, src/glaGen.jl:574-576) for
-//      the 24 face pairs that feed the six stored components, the region heap
-//      of each warp in global scratch;
+//      for the 24 face pairs that feed the six stored components the adaptive
+//      Genz-Malik degree-7/5 cubature (the algorithm of Cubature.jl's
+//      hcubature, src/glaGen.jl:574-576): the rule once per pair and thread,
+//      then a warp for each pair that needs more regions;
 //   4. external operators: circulant separations by grdSel/sepGrd
 //      (src/glaGen.jl:603-645), touching offsets averaged from the contact
 //      self circulant (egoCntOut!, src/glaGen.jl:250-306);
