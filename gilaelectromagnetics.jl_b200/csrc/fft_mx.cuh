@@ -72,28 +72,30 @@ constexpr int mx_inv_mod(int a, int m) {  // a^-1 mod m
   return 1;
 }
 
+// A first: where it is 2 or 4 its inputs are N / A apart, so on a zero-padded
+// line its additions are of exact zeros (B first rounds once more there).
 template <int A, int B, bool INV> struct DftPfa {  // R = A * B, coprime
   template <typename V> GILA_HD static void run(V* v) {
     constexpr int N = A * B;
     constexpr int ca = B * mx_inv_mod(B % A, A) % N, cb = A * mx_inv_mod(A % B, B) % N;
     V t[N];
 #pragma unroll
-    for (int i = 0; i < A; ++i) {
-      V u[B];
-#pragma unroll
-      for (int j = 0; j < B; ++j) u[j] = v[(B * i + A * j) % N];
-      Dft<B, INV>::run(u);
-#pragma unroll
-      for (int j = 0; j < B; ++j) t[i * B + j] = u[j];
-    }
-#pragma unroll
     for (int j = 0; j < B; ++j) {
       V u[A];
 #pragma unroll
-      for (int i = 0; i < A; ++i) u[i] = t[i * B + j];
+      for (int i = 0; i < A; ++i) u[i] = v[(B * i + A * j) % N];
       Dft<A, INV>::run(u);
 #pragma unroll
-      for (int i = 0; i < A; ++i) v[(ca * i + cb * j) % N] = u[i];
+      for (int i = 0; i < A; ++i) t[i * B + j] = u[i];
+    }
+#pragma unroll
+    for (int i = 0; i < A; ++i) {
+      V u[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) u[j] = t[i * B + j];
+      Dft<B, INV>::run(u);
+#pragma unroll
+      for (int j = 0; j < B; ++j) v[(ca * i + cb * j) % N] = u[j];
     }
   }
 };
@@ -111,12 +113,13 @@ template <bool INV> struct Dft<2, INV> {
 template <bool INV> struct Dft<3, INV> {
   template <typename V> GILA_HD static void run(V* v) {
     using T = typename MxOf<V>::T;
+    const T s = (T)0.86602540378443864676372317075293618347;
     const V t = vadd(v[1], v[2]);
     const V m = vfma(t, (T)-0.5, v[0]);
-    const V w = vscale(vmi<INV>(vsub(v[1], v[2])), (T)0.86602540378443864676372317075293618347);
+    const V u = vmi<INV>(vsub(v[1], v[2]));
     v[0] = vadd(v[0], t);
-    v[1] = vadd(m, w);
-    v[2] = vsub(m, w);
+    v[1] = vfma(u, s, m);
+    v[2] = vfma(u, -s, m);
   }
 };
 template <bool INV> struct Dft<4, INV> {
@@ -179,13 +182,13 @@ template <bool INV> struct Dft<8, INV> {
     V e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
     Dft<4, INV>::run(e);
     Dft<4, INV>::run(o);
-    o[1] = vscale(vadd(o[1], vmi<INV>(o[1])), h);
+    o[1] = vadd(o[1], vmi<INV>(o[1]));
     o[2] = vmi<INV>(o[2]);
-    o[3] = vscale(vsub(vmi<INV>(o[3]), o[3]), h);
+    o[3] = vsub(vmi<INV>(o[3]), o[3]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      v[k] = vadd(e[k], o[k]);
-      v[k + 4] = vsub(e[k], o[k]);
+      v[k] = k % 2 ? vfma(o[k], h, e[k]) : vadd(e[k], o[k]);
+      v[k + 4] = k % 2 ? vfma(o[k], -h, e[k]) : vsub(e[k], o[k]);
     }
   }
 };
@@ -384,22 +387,24 @@ template <int P, int KIND> constexpr int mx_line_len() {
   return r0 % 2 == 0 ? P + P / r0 : P;
 }
 // ----------------------------------------------------------------- stages
-// Twiddles q = 1 .. R-1 of a stage of span NS from its table (at jm).  FP64:
-// every fourth loaded, the others one product away from those (two for w^3):
-// a load costs as much of the load/store pipe as a data access.  FP32: all
-// loaded.
-template <int R, int NS, bool INV, typename W>
-__device__ __forceinline__ void mx_twiddles(const W* __restrict__ tw, W* w) {
-  if constexpr (sizeof(W) == 16) {
-    if constexpr (R > 1) w[1] = twid<INV>(tw, 0);
-    if constexpr (R > 2) w[2] = cmul(w[1], w[1]);
-    if constexpr (R > 3) w[3] = cmul(w[2], w[1]);
+// Twiddles q = 1 .. R-1 of a stage of span NS from its table (at jm), all
+// loaded.  In FP64, three of four as products of the others are faster (one
+// product at 80x80x40 0.110 against 0.122 ms, 80x80x50 0.140 / 0.147, 80x80x120
+// 0.351 / 0.380) but carry the products' roundings: relative error of a product
+// at 54x42x36 5.6e-16 against 4.8e-16, at 100x84x60 4.7e-16 against 4.3e-16
+// (runtime-planned kernels: 5.0e-16 and 4.5e-16).
+template <bool INV, typename W> GILA_HD W mx_tw(const W* __restrict__ tw, int m) {
+#ifdef __CUDA_ARCH__
+  W w = __ldg(tw + m);
+#else
+  W w = tw[m];
+#endif
+  if constexpr (INV) w.y = -w.y;
+  return w;
+}
+template <int R, int NS, bool INV, typename W> GILA_HD void mx_twiddles(const W* __restrict__ tw, W* w) {
 #pragma unroll
-    for (int q = 4; q < R; ++q) w[q] = q % 4 == 0 ? twid<INV>(tw, (q - 1) * NS) : cmul(w[q - q % 4], w[q % 4]);
-  } else {
-#pragma unroll
-    for (int q = 1; q < R; ++q) w[q] = twid<INV>(tw, (q - 1) * NS);
-  }
+  for (int q = 1; q < R; ++q) w[q] = mx_tw<INV>(tw, (q - 1) * NS);
 }
 
 // Stage S of a line shared by TPB threads (this thread: j0 of them).  ld(k, i)
