@@ -2501,13 +2501,13 @@ cudaError_t launch_xfwd(const Geom& g, const DevOp<C>& d, const Launch& L, const
 
 template <typename C, bool INV>
 static cudaError_t launch_y_one(const YParams<C>& p, bool mx, int T, size_t sm, int64_t blocks, bool rev, bool gform,
-                                cudaStream_t st) {
+                                bool pairs, cudaStream_t st) {
   if (ct_has_xy(p.P)) {
 #define GILA_CT_Y2(n, tx)                                  \
   if constexpr (ct_y_ok(sizeof(C), n, tx)) {               \
     if (p.P == n && p.TX == tx) {                          \
       if constexpr (sizeof(C) == 8) {                      \
-        if (zpair()) {                                     \
+        if (pairs) {                                       \
           const int T2 = ct_threads2(tx, n);               \
           if (xyg() && gform && (INV ? 2 * p.nout <= n : 2 * p.nin <= n)) { \
             if (rev) {                                     \
@@ -2578,11 +2578,13 @@ static bool chunk_y_tiles(int Px, int txz, int txy, const KxChunk& ch, int& lo0,
   return true;
 }
 
-// ComplexF32 y and z passes move line pairs: even rows on 16-byte boundaries
-// (always so in the operators' own workspaces; a slab piece's caller may
-// hold its planes on any element boundary)
+// Whether the y and z passes may move 16-byte elements: always in ComplexF64;
+// in ComplexF32, where an element is a line pair, on even rows on 16-byte
+// boundaries (always so in the operators' own workspaces; a slab piece's caller
+// may hold its planes on any element boundary).  Elsewhere the tuned lengths
+// run their one-line kernels, the others the runtime-planned ones.
 template <typename C>
-static bool mx_pairs_ok(int Px, const void* a, const void* b) {
+static bool pairs_ok(int Px, const void* a, const void* b) {
   return sizeof(C) == 16 || (Px % 2 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 == 0);
 }
 
@@ -2633,7 +2635,8 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
   p.src_sub = src_sub;
   p.dst_sub = dst_sub;
   if (ct_has_xy(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.y_tx, false);
-  const MxOps<C>* const mx = !ct_has_xy(p.P) && mx_pairs_ok<C>(p.Px, src, dst) ? mx_ops<C>(p.P) : nullptr;
+  const bool pairs = pairs_ok<C>(p.Px, src, dst);
+  const MxOps<C>* const mx = !ct_has_xy(p.P) && pairs ? mx_ops<C>(p.P) : nullptr;
   if (mx) p.TX = mx->y_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
   p.md = make_fdiv((uint32_t)p.TX);
@@ -2649,8 +2652,8 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
   const size_t sm = (size_t)p.TX * p.P * sizeof(C);
   const bool mixed = is_mixed(d.plan[1]);
   const int64_t blocks = (int64_t)p.nt * nq;
-  cudaError_t e = inv ? launch_y_one<C, true>(p, mixed, T, sm, blocks, L.y_rev != 0, L.xy_g != 0, st)
-                      : launch_y_one<C, false>(p, mixed, T, sm, blocks, L.y_rev != 0, L.xy_g != 0, st);
+  cudaError_t e = inv ? launch_y_one<C, true>(p, mixed, T, sm, blocks, L.y_rev != 0, L.xy_g != 0, pairs && zpair(), st)
+                      : launch_y_one<C, false>(p, mixed, T, sm, blocks, L.y_rev != 0, L.xy_g != 0, pairs && zpair(), st);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -2694,7 +2697,8 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
     p.ax[k].fo = (g.tc[k] + 1) / 2;
   }
   if (ct_has(p.P)) p.TX = ct_tile_pick(sizeof(C), p.P, L.z_tx, true);
-  const MxOps<C>* const mx = g.parT == 1 && mx_pairs_ok<C>(p.Px, B, B) ? mx_z<C>(p.P) : nullptr;
+  const bool pairs = pairs_ok<C>(p.Px, B, B);
+  const MxOps<C>* const mx = g.parT == 1 && pairs ? mx_z<C>(p.P) : nullptr;
   if (mx) p.TX = mx->z_tx;
   p.ntiles = (p.Px + p.TX - 1) / p.TX;
   p.md = make_fdiv((uint32_t)p.TX);
@@ -2732,7 +2736,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
       if constexpr (zf_ok(sizeof(C), n)) {            \
         if (p.parT == 1 && zfuse()) {                 \
           if constexpr (sizeof(C) == 8 && zg_ok<n>()) { \
-            if (zpair() && zgo() && 2 * p.nin <= n && 2 * p.nout <= n) { \
+            if (pairs && zpair() && zgo() && 2 * p.nin <= n && 2 * p.nout <= n) { \
               const int T2 = ct_threads2(tx, n);      \
               const void* fn2 = (const void*)k_zg2_ct<n, tx>; \
               cudaError_t e2 = set_smem(fn2, sm);     \
@@ -2741,7 +2745,7 @@ cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, in
             }                                         \
           }                                           \
           if constexpr (sizeof(C) == 8) {             \
-            if (zpair()) {                            \
+            if (pairs && zpair()) {                   \
               const int T2 = ct_threads2(tx, n);      \
               const void* fn2 = (const void*)k_zf2_ct<n, tx>; \
               cudaError_t e2 = set_smem(fn2, sm);     \
