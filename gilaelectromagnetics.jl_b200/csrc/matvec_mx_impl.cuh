@@ -42,10 +42,24 @@ constexpr int mx_blocks(int T, int regs) {
 #ifndef GILA_MX_REGS
 #define GILA_MX_REGS 96
 #endif
-// z pass: up to 84 registers at the short lengths, whose radices stop at 10
-// (50x40x30: 22.2 -> 20.5 us F64, 18.3 -> 16.0 us F32), 104 above (72 and 84
-// spill there: 180x140x90 F32 326 -> 441 us)
-constexpr int mx_z_regs(int P) { return P <= 100 ? 84 : 104; }
+// z pass, by length and last radix RL (a thread of the fused stage holds three
+// components of RL values and a frequency's kernel values):
+// - up to 100, RL 4 (28, 32, 36, 40): 128.  At 84 and 104 these spill 390 and
+//   230 bytes in F64, 480 and 290 in F32: 80x80x20 F64 41.8 and 37.9 us, 29.7 at
+//   128, F32 29.3 and 25.2, 22.9; 80x80x14 F64 33.7 and 29.9, 25.6; at 168 within
+//   4% of 128 either way.
+// - up to 100, RL 2 or 3: 84, two blocks more per SM than 104: 80x80x30 F64 49.3
+//   against 55.4 us, 80x80x50 73.7 / 86.2, 80x80x24 41.5 / 47.8 (54 the exception,
+//   59.6 / 55.5).
+// - above 100: 104.  84 there: 80x80x56 F64 89 -> 100 us, 80x80x80 136 -> 186,
+//   80x80x140 (RL 4) 293 -> 399; 108, 168 and 200 are faster at 84 (168: 192 ->
+//   149), 126 and 252 in F64 not (116 -> 125).
+// (350, 486 and 490 run 648 to 840 threads a block, which the register file
+// holds at 72 to 80 a thread whatever is asked for.)
+template <int P> constexpr int mx_z_regs() {
+  constexpr int RL = mx_r<P, MXK_Z, false>(MxPlan<P, MXK_Z>::s.n - 1);
+  return P > 100 ? 104 : RL == 4 ? 128 : 84;
+}
 // the next frequency's kernel values in flight while one is multiplied: F64
 // above 100 (180x140x90: 613 -> 598 us); elsewhere the registers count for more
 // (F32 180x140x90 345 -> 326 us without)
@@ -262,7 +276,7 @@ struct MxCol {
 };
 
 template <typename C, int P>
-__global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>(), mx_z_regs(P)))
+__global__ void __launch_bounds__(mx_z_threads<P>(), mx_blocks(mx_z_threads<P>(), mx_z_regs<P>()))
     k_z_mx(const ZParams<C> p) {
   using V = typename MxElem<C>::V;
   using W = C;
