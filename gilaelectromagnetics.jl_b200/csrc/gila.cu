@@ -608,7 +608,11 @@ static gila_status tune_on(Core& c, const Geom& g, int64_t nrhs, const C* din, C
   }
   // y tile width jointly with the form of the x / y passes (first stage fed
   // from global memory, or staged through shared memory: the same
-  // arithmetic, the faster one depends on length and precision)
+  // arithmetic, the faster one depends on length and precision); where y has
+  // no tile variants but x has both forms, the form alone (x and y forward at y
+  // length 96, 64x48x32 F64: 18.7 us fed from global memory, 17.7 staged; at 192,
+  // 64x96x48: 29.8 and 30.9)
+  if (yc.empty() && !ct_tiles(cs, c.geom.P[0], false).empty()) yc.push_back(best.y_tx);
   if (!yc.empty() && e == cudaSuccess) {
     float bt = 1e30f;
     int pick = best.y_tx, pick_g = best.xy_g;
