@@ -581,7 +581,7 @@ static gila_status tune_on(Core& c, const Geom& g, int64_t nrhs, const C* din, C
     best.x_rev = keep_radix->x_rev;
     best.y_rev = keep_radix->y_rev;
   }
-  std::vector<int> zc = ct_tiles(cs, c.geom.P[2], true), yc = ct_tiles(cs, c.geom.P[1], false);
+  std::vector<int> zc = z_tiles<C>(c.geom), yc = ct_tiles(cs, c.geom.P[1], false);
   // z tile width jointly with the task form of the fused z pass (one task
   // per thread slot, or one per mirror pair of z frequencies where the
   // kernel has that form; the same arithmetic either way)
@@ -1363,7 +1363,9 @@ gila_status gila_opr_set_tiles(gila_opr* opr, const int32_t tiles[4]) {
   Launch L = c.tuned ? c.launch : default_launch(c);
   const int cs = (int)csize(c.dtype);
   if (tiles[2] > 0) L.y_tx = ct_tile_pick(cs, c.geom.P[1], tiles[2], false) == tiles[2] ? tiles[2] : L.y_tx;
-  if (tiles[3] > 0) L.z_tx = ct_tile_pick(cs, c.geom.P[2], tiles[3], true) == tiles[3] ? tiles[3] : L.z_tx;
+  const std::vector<int> zt = c.dtype == GILA_C128 ? z_tiles<double2>(c.geom) : z_tiles<float2>(c.geom);
+  if (tiles[3] > 0 && (!zt.empty() || ct_tiles(cs, c.geom.P[2], true).empty()))
+    L.z_tx = ct_tile_pick(cs, c.geom.P[2], tiles[3], true) == tiles[3] ? tiles[3] : L.z_tx;
   c.launch = L;
   c.tuned = true;
   c.pinned = true;

@@ -161,6 +161,9 @@ int pass_threads(const AxisPlan& pl, int M);
 // P has no specialised kernels.  ct_tile_pick returns `want` when it is one
 // of them, else the default (128-byte rows, or the widest that fits).
 std::vector<int> ct_tiles(int cs, int P, bool z);
+// z tile widths an operator's z pass can take (empty: one fixed width)
+template <typename C>
+std::vector<int> z_tiles(const Geom& g);
 int ct_tile_pick(int cs, int P, int want, bool z);
 
 }  // namespace gila

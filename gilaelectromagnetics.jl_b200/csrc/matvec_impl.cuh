@@ -2589,12 +2589,18 @@ static bool pairs_ok(int Px, const void* a, const void* b) {
 }
 
 // The length's mixed-radix z pass, or nullptr where the tuned kernels run.
-// ComplexF32 at 64: 45 us in the tuned line-pair kernel, whose last radix 8
-// fills the registers, 38 us with the mixed-radix one's 8 4 2 (two vectors of
-// 64x64x32).
+// ComplexF32 at 64 (unless a switch asks for a form of the tuned kernels): 45 us
+// in the tuned line-pair kernel, whose last radix 8 fills the registers, 38 us
+// with the mixed-radix one's 8 4 2 (two vectors of 64x64x32).
 template <typename C>
 static const MxOps<C>* mx_z(int P) {
-  return !ct_has(P) || (sizeof(C) == 8 && P == 64) ? mx_ops<C>(P) : nullptr;
+  return !ct_has(P) || (sizeof(C) == 8 && P == 64 && zpair() && zfuse() && zgo()) ? mx_ops<C>(P) : nullptr;
+}
+// z tile widths to choose from: none where the mixed-radix pass runs, whose
+// width is fixed
+template <typename C>
+std::vector<int> z_tiles(const Geom& g) {
+  return g.parT == 1 && mx_z<C>(g.P[2]) ? std::vector<int>() : ct_tiles(sizeof(C), g.P[2], true);
 }
 // kx columns per tile of a specialised z pass
 template <typename C>
@@ -3018,6 +3024,7 @@ cudaError_t launch_matvec(const Geom& g, const DevOp<C>& d, const Launch& L, con
                                    int64_t, int64_t, int64_t, cudaStream_t, const KxChunk*);                      \
   template cudaError_t launch_z<C>(const Geom&, const DevOp<C>&, const Launch&, C*, int, cudaStream_t,            \
                                    const KxChunk*, int, int);                                                     \
+  template std::vector<int> z_tiles<C>(const Geom&);                                                              \
   template int kx_chunks<C>(const Geom&, const DevOp<C>&, const Launch&, int);                                    \
   template cudaError_t launch_xinv<C>(const Geom&, const DevOp<C>&, const Launch&, const C*, C*, int64_t,         \
                                       int64_t, bool, C, C, cudaStream_t, const LsEpi<C>*);
