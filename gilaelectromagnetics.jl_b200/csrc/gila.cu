@@ -388,16 +388,19 @@ gila_status init_core(gila_ctx* ctx, const gila_vol* trg_abi, const gila_vol* sr
   GILA_CUDA_TRY(dev_malloc(&core->plan_d, 3 * sizeof(AxisPlan)));
   GILA_CUDA_TRY(cudaMemcpy(core->plan_d, core->plan, 3 * sizeof(AxisPlan), cudaMemcpyHostToDevice));
   GILA_CUDA_TRY(cudaStreamCreateWithFlags(&core->stream, cudaStreamNonBlocking));
-  // the kx-chunk pipeline's streams and events only where it is asked for
-  // (0.5 ms of creating and destroying an operator)
-  const char* const kx = getenv("GILA_KX_CHUNKS");
-  if (!kx || atoi(kx) < 2) return GILA_OK;
-  for (int k = 0; k < 2; ++k) GILA_CUDA_TRY(cudaStreamCreateWithFlags(&core->pipe_st[k], cudaStreamNonBlocking));
-  for (int k = 0; k < kMaxKxChunks; ++k) {
-    GILA_CUDA_TRY(cudaEventCreateWithFlags(&core->pipe_ev_y[k], cudaEventDisableTiming));
-    GILA_CUDA_TRY(cudaEventCreateWithFlags(&core->pipe_ev_z[k], cudaEventDisableTiming));
-  }
-  GILA_CUDA_TRY(cudaEventCreateWithFlags(&core->pipe_join, cudaEventDisableTiming));
+  // (unset, the setting is not looked up yet: it is read at the first matvec)
+  return getenv("GILA_KX_CHUNKS") ? ensure_pipe(*core) : GILA_OK;
+}
+
+gila_status ensure_pipe(Core& c) {
+  if (kx_chunks_wanted() < 2) return GILA_OK;
+  std::lock_guard<std::mutex> lk(c.pipe_mu);
+  for (cudaStream_t& s : c.pipe_st)
+    if (!s) GILA_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  for (int k = 0; k < kMaxKxChunks; ++k)
+    for (cudaEvent_t* ev : {&c.pipe_ev_y[k], &c.pipe_ev_z[k]})
+      if (!*ev) GILA_CUDA_TRY(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+  if (!c.pipe_join) GILA_CUDA_TRY(cudaEventCreateWithFlags(&c.pipe_join, cudaEventDisableTiming));
   return GILA_OK;
 }
 
@@ -494,6 +497,8 @@ Launch default_launch(const Core& c) {
 }
 
 gila_status ensure_work(Core& c, int64_t nrhs) {
+  const gila_status ps = ensure_pipe(c);
+  if (ps != GILA_OK) return ps;
   if (nrhs <= c.cap_rhs) return GILA_OK;
   c.geom.max_rhs = (int)nrhs;
   const Work w = work_sizes(c.geom);
@@ -1406,7 +1411,10 @@ gila_status gila_opr_device_bytes(const gila_opr* opr, int64_t* bytes) {
 
 gila_status gila_opr_launches_per_apply(const gila_opr* opr, int64_t nrhs, int64_t* n) {
   if (!opr || !n || nrhs < 1) return fail(GILA_ERR_ARG, "invalid argument");
-  const Core& c = *opr->core;
+  Core& c = *opr->core;
+  GILA_CUDA_TRY(cudaSetDevice(c.device));
+  const gila_status s = ensure_pipe(c);
+  if (s != GILA_OK) return s;
   Geom g = c.geom;
   if (nrhs > g.max_rhs) g.max_rhs = (int)nrhs;
   const Launch L = c.tuned ? c.launch : default_launch(c);

@@ -95,8 +95,9 @@ struct Core {
   bool pinned = false;    // launch shapes forced by the caller (set_tiles / set_schedule)
   cudaStream_t stream = nullptr;
   // the kx-chunk pipeline of the matvec (matvec.cuh): z-pass and inverse-y
-  // streams and their events, made with the operator so that no apply or
-  // stream capture creates any
+  // streams and their events, made where it is asked for (ensure_pipe): 0.5 ms
+  // of creating and destroying an operator
+  std::mutex pipe_mu;
   cudaStream_t pipe_st[2] = {nullptr, nullptr};
   cudaEvent_t pipe_ev_y[kMaxKxChunks] = {}, pipe_ev_z[kMaxKxChunks] = {};
   cudaEvent_t pipe_join = nullptr;
@@ -125,6 +126,9 @@ Launch default_launch(const Core& c);
 // GPU FP64 Fourier-kernel build into c.ker (kerbuild.cu)
 gila_status build_kernel(Core& c);
 gila_status ensure_work(Core& c, int64_t nrhs);
+// the kx-chunk pipeline's streams and events if GILA_KX_CHUNKS asks for it, for
+// every path that runs whole matvecs, ahead of its launches and captures
+gila_status ensure_pipe(Core& c);
 void release_work(Core& c);  // frees the matvec workspaces (allocated again on demand)
 // launch shapes: cached per context, else timed (autotune) at first use
 gila_status ensure_tuned(Core& c, int64_t nrhs);

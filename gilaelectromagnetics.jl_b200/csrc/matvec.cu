@@ -20,6 +20,7 @@
 //          scatter (mrgPrtDev!, src/glaActSup.jl:956-1004) and the mul!
 //          axpby epilogue (src/glaLinAlg.jl:61-69) fused into the store.
 #include <cstdio>
+#include <cstdlib>
 
 #include "fft_ct.cuh"
 #include "matvec.cuh"
@@ -78,6 +79,15 @@ int64_t matvec_launches(const Geom& g, int nrhs, int kx_chunks) {
   const int64_t nf = fwd_flat ? slabs(fwd_planes * nrhs) : nrhs * slabs(fwd_planes);
   const int64_t ni = inv_flat ? slabs(inv_planes * nrhs) : nrhs * slabs(inv_planes);
   return 2 * nf + 1 + 2 * ni;
+}
+
+int kx_chunks_wanted() {
+  static const int n = [] {
+    const char* e = getenv("GILA_KX_CHUNKS");
+    const int v = e ? atoi(e) : 0;
+    return v < 0 ? 0 : (v > kMaxKxChunks ? kMaxKxChunks : v);
+  }();
+  return n;
 }
 
 static bool ct_len(int P) {

@@ -133,6 +133,8 @@ cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv
 template <typename C>
 cudaError_t launch_z(const Geom& g, const DevOp<C>& d, const Launch& L, C* B, int nrhs, cudaStream_t st,
                      const KxChunk* ch = nullptr, int ky0 = 0, int nky = -1);
+// GILA_KX_CHUNKS, read once per process
+int kx_chunks_wanted();
 // kx chunks the pipelined matvec uses for this operator and launch shape
 // (0: no pipeline)
 template <typename C>

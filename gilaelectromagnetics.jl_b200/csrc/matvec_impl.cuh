@@ -2609,6 +2609,13 @@ static int z_tile(int P, int want) {
   return o ? o->z_tx : ct_tile_pick(sizeof(C), P, want, true);
 }
 
+// kx columns per tile of the y pass at a tuned or mixed-radix length
+template <typename C>
+static int y_tile(int P, int want) {
+  const MxOps<C>* const o = ct_has_xy(P) ? nullptr : mx_ops<C>(P);
+  return o ? o->y_tx : ct_tile_pick(sizeof(C), P, want, false);
+}
+
 template <typename C>
 cudaError_t launch_y(const Geom& g, const DevOp<C>& d, const Launch& L, bool inv, const C* src, C* dst, int64_t q0,
                      int64_t nq, int64_t src_sub, int64_t dst_sub, cudaStream_t st, const KxChunk* ch) {
@@ -2941,25 +2948,15 @@ cudaError_t launch_matvec_phase(int phase, const Geom& g, const DevOp<C>& d, con
 // self operators with specialised y / z lengths, one target partition, the
 // x/y slab holding every plane of every vector, chunk boundaries on both
 // tile widths
-static inline int kx_chunks_wanted() {
-  static const int n = [] {
-    const char* e = getenv("GILA_KX_CHUNKS");
-    const int v = e ? atoi(e) : 0;
-    return v < 0 ? 0 : (v > kMaxKxChunks ? kMaxKxChunks : v);
-  }();
-  return n;
-}
-
 template <typename C>
 int kx_chunks(const Geom& g, const DevOp<C>& d, const Launch& L, int nrhs) {
   const int want = kx_chunks_wanted();
   if (want < 2 || !d.pst[0] || !d.pst[1] || !d.pjoin || g.parT != 1) return 0;
-  if (!ct_has_xy(g.P[1]) || !ct_has(g.P[2])) return 0;
+  if (!ct_has(g.P[1]) || !ct_has(g.P[2])) return 0;
   const Work w = work_sizes(g);
   const int64_t fwd = 3LL * g.sc[2] * nrhs, inv = 3LL * g.tc[2] * nrhs;
   if ((int64_t)w.zb != g.sc[2] || (int64_t)w.zb != g.tc[2] || w.slab_planes < fwd || w.slab_planes < inv) return 0;
-  const int txz = z_tile<C>(g.P[2], L.z_tx);
-  const int txy = ct_tile_pick(sizeof(C), g.P[1], L.y_tx, false);
+  const int txz = z_tile<C>(g.P[2], L.z_tx), txy = y_tile<C>(g.P[1], L.y_tx);
   const int Px = g.P[0];
   if (Px % txz || Px % txy || (Px / txz) % 2) return 0;
   const int pairs = Px / txz / 2;

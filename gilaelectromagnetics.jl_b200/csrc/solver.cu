@@ -670,6 +670,10 @@ class LsBatchT final : public LsBatch {
   gila_status init() {
     GILA_CUDA_TRY(cudaStreamCreateWithPriority(&s_, cudaStreamNonBlocking, cfg_.priority));
     GILA_CUDA_TRY(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
+    for (Core* c : {&g64_, &gi_}) {
+      const gila_status ps = ensure_pipe(*c);
+      if (ps != GILA_OK) return ps;
+    }
     const size_t vb = (size_t)S_ * n_;
     const bool mixed = cfg_.mixed != 0;
     const int nchi = cfg_.chi_shared ? 1 : S_;
