@@ -318,11 +318,13 @@ constexpr MxSched mx_search(int P, int rmax, int last_max, int stage_cost) {
 // MXK_XY: x and y passes; MXK_Z: fused z pass, whose last radix three
 // components share a thread's registers
 enum { MXK_XY = 0, MXK_Z = 1 };
-#ifndef GILA_MX_STAGE
-#define GILA_MX_STAGE 400
-#endif
+// Radices up to 10 to length 100, where larger ones gain at some lengths (z 72 at
+// 80x80 F64 62.6 -> 54.0 us, 84 76.6 -> 68.4) and lose at others and at small
+// volumes (x and y 80 at 40x40x64 34.6 -> 45.3 us, F32 27.5 -> 39.5); up to 16
+// above, where 10 loses (z 112 at 80x80 F64 90 -> 133 us, 140 119 -> 165; x and y
+// 120 at 60x60x64 48.5 -> 58.5 us).
 constexpr MxSched mx_sched(int P, int kind) {
-  return mx_search(P, P <= 100 ? 10 : 16, kind == MXK_Z ? 4 : 16, GILA_MX_STAGE);
+  return mx_search(P, P <= 100 ? 10 : 16, kind == MXK_Z ? 4 : 16, 400);
 }
 template <int P, int KIND> struct MxPlan {
   static constexpr MxSched s = mx_sched(P, KIND);

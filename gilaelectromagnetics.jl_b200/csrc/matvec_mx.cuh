@@ -1,9 +1,9 @@
 // matvec_mx.cuh -- the mixed-radix passes: launch table by transform length.
 //
 // Every even length 2^a 3^b 5^c 7^d from 4 to 512 that fft_ct.cuh does not
-// specialise has compile-time kernels here (matvec_mx_impl.cuh; 96, 192 and 384
-// the x and y ones); longer lengths and the z pass of target partitions keep
-// the runtime-planned kernels.
+// specialise has compile-time kernels here (matvec_mx_impl.cuh), 96, 192 and 384
+// the x and y ones, 64 the ComplexF32 z one; longer lengths and the z pass of
+// target partitions keep the runtime-planned kernels.
 #pragma once
 #include "passes.cuh"
 
@@ -15,10 +15,12 @@ template <typename C>
 struct MxOps {
   int P;
   int y_tx, z_tx;  // kx columns per tile of the y and z passes
+  // null where the tuned kernels are the faster: x and y at 64, z at 96, 192,
+  // 384 and in ComplexF64 at 64
   cudaError_t (*xfwd)(const XfParams<C>&, cudaStream_t);
   cudaError_t (*xinv)(const XiParams<C>&, bool axpby, cudaStream_t);
   cudaError_t (*y)(const YParams<C>&, bool inv, int64_t units, cudaStream_t);
-  cudaError_t (*z)(const ZParams<C>&, int64_t blocks, cudaStream_t);  // null at 96, 192, 384
+  cudaError_t (*z)(const ZParams<C>&, int64_t blocks, cudaStream_t);
 };
 
 // the length's launches, or nullptr where it has none; the lengths are spread

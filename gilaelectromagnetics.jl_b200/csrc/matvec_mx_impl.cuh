@@ -39,9 +39,7 @@ constexpr int mx_blocks(int T, int regs) {
   const int b = 65536 / (mx_up32(T) * regs);
   return b < 1 ? 1 : (b > 16 ? 16 : b);
 }
-#ifndef GILA_MX_REGS
-#define GILA_MX_REGS 96
-#endif
+constexpr int kMxRegs = 96;  // y pass
 // z pass, by length and last radix RL (a thread of the fused stage holds three
 // components of RL values and a frequency's kernel values):
 // - up to 100, RL 4 (28, 32, 36, 40): 128.  At 84 and 104 these spill 390 and
@@ -214,7 +212,7 @@ template <int P> constexpr int mx_y_units() {
 template <int P> constexpr int mx_y_threads() { return mx_y_units<P>() * kMxTX * MxPlan<P, MXK_XY>::s.tpb; }
 
 template <typename C, int P, bool INV>
-__global__ void __launch_bounds__(mx_y_threads<P>(), mx_blocks(mx_y_threads<P>(), GILA_MX_REGS))
+__global__ void __launch_bounds__(mx_y_threads<P>(), mx_blocks(mx_y_threads<P>(), kMxRegs))
     k_y_mx(const YParams<C> p, const uint32_t units) {
   using V = typename MxElem<C>::V;
   constexpr int TX = kMxTX, CW = 16 / sizeof(C), TPB = MxPlan<P, MXK_XY>::s.tpb, NU = mx_y_units<P>();
@@ -250,10 +248,7 @@ __global__ void __launch_bounds__(mx_y_threads<P>(), mx_blocks(mx_y_threads<P>()
 // -------------------------------------------------------------------- z
 // kx elements per tile: 128-byte rows while three components' lines leave
 // room for two blocks or more per SM, else half of that
-#ifndef GILA_MX_ZTX8
-#define GILA_MX_ZTX8 192
-#endif
-template <int P> constexpr int mx_z_tx() { return P <= GILA_MX_ZTX8 ? 8 : 4; }
+template <int P> constexpr int mx_z_tx() { return P <= 192 ? 8 : 4; }
 // z lines of a tile in shared memory: rows of TX elements, at tiles of 4 padded
 // like an x line (two rows share a quarter-warp's banks)
 template <int P> GILA_HD int mx_z_row(int i) { return mx_z_tx<P>() == 8 ? i : mx_pad<P, MXK_Z>(i); }
@@ -508,13 +503,26 @@ struct MxLaunch {
     if (e != cudaSuccess) return e;
     return launch_pass(k_z_mx<C, P>, (unsigned)blocks, mx_z_threads<P>(), sm, st, p);
   }
-  static constexpr auto z_or_null() -> decltype(&z) {
-    if constexpr (P == 96 || P == 192 || P == 384)
-      return nullptr;
-    else
-      return &z;
+  // launches that the dispatch can reach: at 96, 192 and 384 the x and y
+  // passes, at 64 the ComplexF32 z pass; every pass elsewhere
+  static constexpr bool XY = P != 64, Z = P == 64 ? sizeof(C) == 8 : !(P == 96 || P == 192 || P == 384);
+  static constexpr auto xfwd_fn() -> decltype(&xfwd) {
+    if constexpr (XY) return &xfwd;
+    return nullptr;
   }
-  static constexpr MxOps<C> ops{P, kMxTX * CW, mx_z_tx<P>() * CW, &xfwd, &xinv, &y, z_or_null()};
+  static constexpr auto xinv_fn() -> decltype(&xinv) {
+    if constexpr (XY) return &xinv;
+    return nullptr;
+  }
+  static constexpr auto y_fn() -> decltype(&y) {
+    if constexpr (XY) return &y;
+    return nullptr;
+  }
+  static constexpr auto z_fn() -> decltype(&z) {
+    if constexpr (Z) return &z;
+    return nullptr;
+  }
+  static constexpr MxOps<C> ops{P, kMxTX * CW, mx_z_tx<P>() * CW, xfwd_fn(), xinv_fn(), y_fn(), z_fn()};
 };
 
 template <typename C, int... P>
