@@ -1103,7 +1103,12 @@ __global__ void __launch_bounds__(256) k_far_first(const FarParams p, const Pair
 // fails.  A pair is a chain of dependent rule evaluations, so its latency
 // counts (near pairs of a cubic cell: 0.81 ms with pass 1's regions in global
 // memory and the two child regions one after the other, 0.53 ms with a
-// half-warp each; 15.3 ms with all 36 pairs of an offset on one warp).
+// half-warp each; 15.3 ms with all 36 pairs of an offset on one warp).  Cubic
+// cells of 1/28 to 1/36 stay below 400 regions; flat and long ones reach pass
+// 2 (cells 1/32 x 1/32 x 1/96: 31 pairs, up to 13,763 regions), whose eight
+// warps take a few rounds: build at 16^3 614 -> 74 ms, 1/32 x 1/32 x 1/64 at
+// 32^3 229 -> 14.5 ms, 1/16 x 1/128 x 1/128 at 16^3 419 -> 47 ms (all 36 pairs
+// of an offset in turn, with a heap, before).
 constexpr int kCap0 = 48, kCap1 = 512, kCap2 = 16384;
 constexpr int kRegBytes = sizeof(Region) + sizeof(double);
 template <bool RF>
@@ -2090,7 +2095,7 @@ gila_status build_kernel(Core& c) {
   int flags[2];
   KB_TRY(cudaMemcpyAsync(flags, err_d, sizeof(flags), cudaMemcpyDeviceToHost, B.st));
   KB_TRY(cudaStreamSynchronize(B.st));
-  if (flags[0]) return fail(GILA_ERR_INTERNAL, "kernel build: cubature region capacity or iteration cap exceeded");
+  if (flags[0]) return fail(GILA_ERR_INTERNAL, "kernel build: cubature region capacity exceeded");
   if (flags[1]) return fail(GILA_ERR_NAN, "Fourier information contains non-numeric values.");
   return GILA_OK;
 }

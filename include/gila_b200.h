@@ -211,10 +211,11 @@ gila_status gila_opr_autotune(gila_opr* opr, int64_t nrhs, int32_t tiles[4]);
 gila_status gila_opr_get_tiles(gila_opr* opr, int32_t tiles[4]);
 gila_status gila_opr_set_tiles(gila_opr* opr, const int32_t tiles[4]);
 
-/* Radix order of the x and y transforms at the specialised lengths (no
- * counterpart in the reference, whose FFTs are FFTW / CUFFT plans): sched =
- * {x, y}, 0 = the greedy order (radix-8 stages first), 1 = its reverse.  Both
- * compute the same transform; results differ by rounding only.  The autotuner
+/* Radix order of the x and y transforms (no counterpart in the reference,
+ * whose FFTs are FFTW / CUFFT plans): sched = {x, y}, 0 = the greedy order
+ * (radix-8 stages first), 1 = its reverse.  Both compute the same transform;
+ * results differ by rounding only.  Lengths 128 and 256 have the two orders; at
+ * every other length the setting is kept and changes nothing.  The autotuner
  * picks them together with the tiles; set forces them (entries < 0 keep the
  * current value). */
 gila_status gila_opr_get_schedule(gila_opr* opr, int32_t sched[2]);
