@@ -214,10 +214,12 @@ __device__ __forceinline__ void pass_begin() {
 
 // A launch of up to kEarlyBlocks blocks may be scheduled before the kernel
 // ahead of it has finished (the kernel starts with pass_begin()): the launch
-// gaps of a product's five kernels, about 1 us each, overlap (16^3 F64 43 -> 35
-// us, 50x40x30 61 -> 54 us, external 64^3 -> 64x64x32 114 -> 104 us, 128x128x64
-// 370 -> 363 us).  Launches of more blocks run for 0.2 ms and longer, where
-// waiting blocks cost more than the gap (256x256x128: 3.347 -> 3.370 ms).
+// gaps of a product's five kernels, about 1 us each, overlap (one product, device
+// time: 16^3 F64 32.7 -> 30.2 us, 50x40x30 52.1 -> 48.9, 128x128x64 369 -> 364,
+// 192x192x96 F32 826 -> 821; 250x196x120 and larger unchanged).  The largest
+// products lose where they follow one another (256x256x128 F64, up to 32768
+// blocks a pass: 3.370 -> 3.403 ms a product with every launch early, 192x192x96
+// F32, up to 9216: unchanged).
 constexpr unsigned kEarlyBlocks = 16384;
 template <typename... KA, typename... A>
 inline cudaError_t launch_pass(void (*k)(KA...), unsigned blocks, int threads, size_t smem, cudaStream_t st, A&&... a) {

@@ -399,8 +399,9 @@ __device__ inline Z block_sum(Z v, Z* sh) {
 // self, 1: edge, 2: vertex), item0 .. item0 + nitems - 1 with `outer` blocks
 // each; partial[item][outer].
 //
-// Bound by FP64 arithmetic: 906 M kernel values for three directions at intOrd
-// 32, a third of that where the sides are equal.  All items of a kind in one
+// Bound by FP64 arithmetic (the pipe at 55 to 63% of its peak) and the latency of
+// its chains at 16 warps or fewer per SM: 906 M kernel values for three directions
+// at intOrd 32, a third of that where the sides are equal.  All items of a kind in one
 // launch: an item alone has 32 (vertex) to 768 blocks, and one after the other
 // they left most SMs idle.  A kernel per kind, with the pair's geometry in
 // shared memory, holds 76 to 128 registers (one kernel for all: 152, one block
@@ -983,10 +984,10 @@ struct Lists {
 
 // Items one block takes at a time.  A thread runs the 57 points of one
 // (item, pair) by itself -- no reductions, and the pairs of a warp differ only
-// in the table column and the separation they read.  Bound by FP64 arithmetic:
-// the warp-per-offset form before it spent its time in the serial sums and
-// the global-memory heap of its one active lane (32^3 cells: 9.0 ms, now 0.26
-// ms and 0.13 ms of k_adapt).
+// in the table column and the separation they read.  The FP64 pipe is at 46% of
+// its peak at a quarter of the warps; the warp-per-offset form before it spent
+// its time in the serial sums and the global-memory heap of its one active lane
+// (32^3 cells: 9.0 ms, now 0.26 ms and 0.13 ms of k_adapt).
 constexpr int kFarItems = 32;
 template <bool RF>
 __global__ void __launch_bounds__(256) k_far_first(const FarParams p, const PairGeo* __restrict__ gp, int64_t item0,

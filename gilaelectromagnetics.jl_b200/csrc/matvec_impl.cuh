@@ -2290,9 +2290,9 @@ __global__ void __launch_bounds__(ct_threads(ct_xlines<sizeof(C)>(P), P)) k_xinv
 // Lengths with specialised kernels.
 #define GILA_CT_SIZES(X) X(64) X(96) X(128) X(192) X(256) X(384) X(512)
 // of them, lengths with x and y kernels: at 96, 192 and 384 the mixed-radix x
-// and y passes are faster (both directions, F64: 0.340 -> 0.296 ms at 192 with
-// four vectors of 96x96x48, 0.786 -> 0.589 ms at 384 with 192x192x96; F32: 0.197
-// -> 0.165 and 0.440 -> 0.374 ms), their z passes slower (0.318 -> 0.454 ms)
+// and y passes are faster (both directions, F64: 0.340 -> 0.304 ms at 192 with
+// four vectors of 96x96x48, 0.786 -> 0.655 ms at 384 with 192x192x96; F32: 0.197
+// -> 0.162 and 0.440 -> 0.367 ms), their z passes slower (0.318 -> 0.454 ms)
 #define GILA_CT_XY_SIZES(X) X(64) X(128) X(256) X(512)
 static bool ct_has_xy(int P) { return P == 64 || P == 128 || P == 256 || P == 512; }
 static bool ct_has(int P) {
@@ -2589,9 +2589,11 @@ static bool pairs_ok(int Px, const void* a, const void* b) {
 }
 
 // The length's mixed-radix z pass, or nullptr where the tuned kernels run.
-// ComplexF32 at 64 (unless a switch asks for a form of the tuned kernels): 45 us
-// in the tuned line-pair kernel, whose last radix 8 fills the registers, 38 us
-// with the mixed-radix one's 8 4 2 (two vectors of 64x64x32).
+// ComplexF32 at 64 (unless a switch asks for a form of the tuned kernels): its
+// last radix 8 fills the tuned line-pair kernel's registers, the mixed-radix one
+// runs 8 4 2.  Tuned -> mixed z pass, 32 cells along z: 8x8 16.9 -> 10.6 us, 32x32
+// 21.5 -> 12.4, 64x64 26.1 -> 22.8, two vectors 44.5 -> 37.1, 128x128 101 -> 68,
+// four vectors 348 -> 243, 250x96 151 -> 100.
 template <typename C>
 static const MxOps<C>* mx_z(int P) {
   return !ct_has(P) || (sizeof(C) == 8 && P == 64 && zpair() && zfuse() && zgo()) ? mx_ops<C>(P) : nullptr;

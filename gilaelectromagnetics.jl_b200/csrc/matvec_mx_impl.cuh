@@ -3,14 +3,14 @@
 //
 // Against the runtime-planned kernels (fft.cuh) that these lengths ran on:
 // index arithmetic, radices and spans are constants, a stage's radix goes up
-// to 10 (two or three shared-memory round trips a line instead of three to
-// five), the first stage is fed from global memory and the last one writes
-// it, ComplexF32 moves line pairs, and the z pass multiplies in registers
-// between its last forward and first inverse butterfly and runs its three
-// components on separate threads.  One product, runtime-planned -> these:
-// 16^3 F64 66 -> 44 us (both with 25 us of host and launch time), 50x40x30
-// F64 157 -> 61 us, 100x84x60 F64 1.115 -> 0.268 ms (1.8 TB/s of the
-// algorithmic bytes), 180x140x90 F32 3.63 -> 0.706 ms (1.6 TB/s).
+// to 10 at lengths to 100 and to 16 above (two or three shared-memory round
+// trips a line instead of three to five), the first stage is fed from global
+// memory and the last one writes it, ComplexF32 moves line pairs, and the z pass
+// multiplies in registers between its last forward and first inverse butterfly
+// and runs its three components on separate threads.  One product as a timed
+// call, runtime-planned -> these: 16^3 F64 66 -> 35 us (25 us of it host), 50x40x30
+// F64 157 -> 53 us, 100x84x60 F64 1.114 -> 0.240 ms (2.0 TB/s of the algorithmic
+// bytes), 180x140x90 F32 3.63 -> 0.585 ms (1.9 TB/s).
 #pragma once
 #include "fft_mx.cuh"
 #include "matvec_mx.cuh"
