@@ -54,6 +54,7 @@ static gila_status noalloc_t(Core& c, const void* in, void* out, cudaStream_t us
   void* scratch = nullptr;
   gila_status s = noalloc_scratch(c.device, &scratch);
   if (s != GILA_OK) return s;
+  if ((s = ensure_pipe(c)) != GILA_OK) return s;  // (nothing unless GILA_KX_CHUNKS is set)
   // Workspace plan: the whole padded spectrum B of one vector, plus an x/y
   // slab A sized to whatever room is left (at least one plane).
   Geom g = c.geom;

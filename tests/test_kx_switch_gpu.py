@@ -17,8 +17,9 @@ from conftest import ROOT
 pytestmark = pytest.mark.gpu
 
 CHILD = r"""
-import json, os, sys
+import ctypes as ct, json, os, sys
 import numpy as np
+import torch
 sys.path.insert(0, {root!r}); sys.path.insert(0, {tests!r})
 from conftest import load_pkg
 from oracle.synth import seeded_current, synth_operator
@@ -40,6 +41,17 @@ for k, (cel, dtype, mem) in enumerate(mems):
     y = np.zeros_like(xs, order="F")
     mem.apply_into(xs, y, nrhs=2)
     out["y%d" % k], n["y%d" % k] = y, mem.launches_per_apply(2)
+# the allocation-free entry point as an operator's first call
+cel = (32, 48, 48)
+mix, fur, *_ = synth_operator(cel, SCL, (0, 0, 0), None, None)
+mem = gila.GlaOprMem(gila.GlaKerOpt(True), gila.GlaVol(cel, SCL), egoFur=fur, setTyp=np.complex128)
+xt = torch.from_numpy(seeded_current(cel, 7).ravel(order="F").copy()).cuda()
+yt = torch.zeros_like(xt)
+torch.cuda.synchronize()
+L = gila._lib
+assert L.lib().gila_opr_apply_noalloc(mem._h, L.GILA_C128, ct.c_void_p(xt.data_ptr()), xt.numel(),
+                                      ct.c_void_p(yt.data_ptr()), yt.numel(), None) == L.GILA_OK
+out["noalloc"] = yt.cpu().numpy()
 chi = np.zeros((32, 48, 32), dtype=np.complex128, order="F")
 chi[8:24, 8:24, 8:24] = 2.0 + 0.1j
 x, info = gila.solve(gila.LippmannSchwinger(G, chi), np.asfortranarray(seeded_current((32, 48, 32), 5)), mixed=True)
